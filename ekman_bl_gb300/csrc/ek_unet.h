@@ -69,6 +69,8 @@ class UNet {
   float *gy_ = nullptr;
   float *gt_[kLevels] = {}, *gs_[kLevels] = {}, *gp_[kLevels] = {};
   float *gu_[kLevels] = {}, *gv_[kLevels] = {}, *gd_[kLevels] = {};
+  // BF16 copies of the gradients that are a layer's dZ
+  unsigned short *gtb_[kLevels] = {}, *gsb_[kLevels] = {}, *gvb_[kLevels] = {}, *gdb_[kLevels] = {};
   double *loss_ = nullptr;
   std::vector<void *> bufs_, gbufs_;
 

@@ -186,3 +186,47 @@ def test_guess_in_solver():
     assert np.mean(cyc_g) <= np.mean(cyc_0), (cyc_g, cyc_0)
     for x_, y_ in zip(a.download(), b.download()):
         assert rel_l2(x_, y_) < 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("C,n,h,w,hv,wv", [(32, 1, 8, 8, 8, 8),          # one partial tile
+                                           (16, 4, 24, 40, 16, 32),      # 16-channel tiles, a ragged last tile
+                                           (32, 2, 16, 264, 16, 256)])   # rows longer than a tile: halo in pieces
+def test_backward_kernels_match_elementwise_gemm(C, n, h, w, hv, wv):
+    """The tensor-core passes against k_conv_gemm's (set_tcgen05 off), which
+    the oracle tests cover.  Weights of a few +-1 an output, small whole
+    inputs and a power-of-two pixel count keep every sum of the forward and
+    input-gradient passes exact in FP32, so both ways give the same values
+    whatever their order: the prediction agrees bit for bit, and the weight
+    and bias gradients are the same products summed over P pixels in another
+    FP32 order, each within about sqrt(P/2) 2^-24 of its size."""
+    import torch
+    from ekman_bl_gb300.duct import UNet
+    rng = np.random.default_rng(7)
+    parts = []
+    for ci, co, *_ in layer_specs(2, C):
+        wt = np.zeros((co, 9 * ci), np.float32)
+        for r in wt:
+            r[rng.choice(9 * ci, 3, replace=False)] = rng.choice([-1, 1, 1], 3)
+        parts += [wt.ravel(), rng.integers(0, 2, co).astype(np.float32)]
+    x = torch.from_numpy(rng.integers(-4, 5, (n, h, w, 2)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.integers(-4, 5, (n, h, w)).astype(np.float32)).cuda()
+    net = UNet(2, C, n, h, w)
+    net.set_params(np.concatenate(parts))
+    out = []
+    for on in (True, False):
+        net.set_tcgen05(on)
+        y = torch.zeros((n, h, w), device="cuda")
+        loss, g = net.gradient(x.data_ptr(), t.data_ptr(), n, hv, wv, y.data_ptr())
+        out.append((y, g))
+    (ya, ga), (yb, gb) = out
+    assert torch.equal(ya, yb) and float(ya.abs().max()) > 0
+    tol = 4 * np.sqrt(n * h * w) * 2.0 ** -24
+    off = used = 0
+    for l, (ci, co, *_) in enumerate(layer_specs(2, C)):
+        for k in (co * 9 * ci, co):
+            a, b = ga[off:off + k], gb[off:off + k]
+            used += bool(np.any(b))
+            assert rel_l2(a, b) <= tol, (l, k, rel_l2(a, b))
+            off += k
+    assert off == ga.size and used >= 20
