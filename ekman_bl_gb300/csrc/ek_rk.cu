@@ -309,7 +309,7 @@ struct AdiArgs {
   // eliminated diagonal and the upper diagonal
   const double *nut, *ltab;
   double *scr_b, *scr_u;
-  // the float-float variant (k_adi_les_ff): NU_T in FP32 and the weights of
+  // the float-float variant (k_adi_les_tile): NU_T in FP32 and the weights of
   // both tables split into float-float planes (0..3 right-hand side, 4..10 row)
   const float *nutf;
   const float2 *ftab;
@@ -549,6 +549,21 @@ __device__ __forceinline__ FF ff_rcp(FF b) {
 __device__ __forceinline__ FF ff2(float2 v) { return FF(v.x, v.y); }
 __device__ __forceinline__ FF ff1(float v) { return FF(v, 0.0f); }
 
+// FF((double)v) on the FP32 pipe: the low part rounded to the 53 bits a double
+// holds.  With hi = 1.m 2^E the sum's last place is 2^(E-52) (one lower when
+// the sum falls below a power of two hi), and a low part under 2^(E-29) loses
+// the bits below it, to nearest even, when a 2^(E-29) of its sign is added and
+// taken away.  Values under 2^-96 keep their low part whole.
+__device__ __forceinline__ FF ff_round53(FF v) {
+  const unsigned uh = __float_as_uint(v.hi), ul = __float_as_uint(v.lo);
+  const unsigned e = uh & 0x7f800000u;
+  const bool below = (uh & 0x7fffffu) == 0u && ((uh ^ ul) >> 31);
+  const unsigned ce = e - ((below ? 30u : 29u) << 23);
+  const float c = __uint_as_float(ce | (ul & 0x80000000u));
+  if (e > (31u << 23) && (ul & 0x7f800000u) < ce) v.lo = __fsub_rn(__fadd_rn(c, v.lo), c);
+  return v;
+}
+
 // The weights of one sweep's two tables split into float-float planes.
 __global__ void k_adi_ff_tab(int n2, const double *rhs_tab, const double *row_tab, float2 *ftab) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -560,128 +575,223 @@ __global__ void k_adi_ff_tab(int n2, const double *rhs_tab, const double *row_ta
   }
 }
 
-// k_adi_les in float-float arithmetic, for the mixed-precision method: the
-// rows, the elimination and the back substitution run on the FP32 pipe at
-// about 46 significant bits; the FP64 pipe only splits the five FP64 inputs
-// of a row and joins the result.  The eliminated rows go to the scratch
-// fields (and the modified right-hand side into the output) as float pairs
-// in the same 8-byte slots.
-template <bool ZS, bool SF>
-__global__ void __launch_bounds__(128) k_adi_les_ff(AdiArgs a) {
+// k_adi_les in float-float arithmetic, for the mixed-precision method (whose
+// explicit part is the FP32 increment S): the rows, the elimination and the
+// back substitution run on the FP32 pipe at about 46 significant bits, and
+// the FP64 pipe only splits the y sweep's three FP64 inputs of a row and joins
+// the z sweep's result.  The y sweep leaves phi* as float pairs in PHS, rounded
+// as an FP64 field would hold it, so the z sweep splits nothing.
+//
+// A block owns 32 x points of one line, lane = x point.  Four warps build the
+// rows, kLesRows at a time, two consecutive rows a turn, into a two-slot ring
+// in shared memory; one warp runs the recurrence (one reciprocal a row,
+// FF chains of ~200 cycles) through the slot built before.  The eliminated
+// rows go to the scratch fields and the output's slots as float pairs, and
+// the back substitution takes them back through the same ring, copied
+// asynchronously a chunk ahead.
+// What bounds it: with one thread a system (the form before this one) a row
+// cost 2.8 us on 256 x 193 x 129, its twenty loads' latency in series with
+// the recurrence at 7 warps an SM; now the loads of kLesRows rows are in
+// flight in four warps while the recurrence works, which leaves the
+// recurrence's own latency and the y sweep's FP64 splits.
+// Measured, the four fields' sweeps of a 256 x 193 x 129 step: y 6.5 -> 3.2 ms,
+// z 5.1 -> 2.2 ms.
+constexpr int kLesRows = 16, kLesWarps = 5;
+
+template <bool ZS>
+__global__ void __launch_bounds__(32 * kLesWarps) k_adi_les_tile(AdiArgs a) {
+  // a row of a lane: (L, D) and (U, V) as float pairs
+  __shared__ float4 ring[2][kLesRows][2][32];
+  __shared__ float2 wts[kLesWarps - 1][2][11];
   const Dims &d = a.d;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = (int)blockIdx.x * 32 + lane;
   const int line = ZS ? (int)blockIdx.y : a.zs + (int)blockIdx.y;
-  if (i >= d.NX) return;
+  const bool on = i < d.NX;
+  const float2 *ps = reinterpret_cast<const float2 *>(a.phs);
+  const double *po = a.phi_old;
   if (ZS && (line < a.js || line > a.je)) {
-    for (int k = a.zs; k <= a.ze; ++k) a.out[d.ip(i, k, line)] = a.phs[d.ip(i, k, line)];
+    if (on)
+      for (int k = a.zs + warp; k <= a.ze; k += kLesWarps) {
+        const size_t q = d.ip(i, k, line);
+        a.out[q] = (double)ff2(ps[q]);
+      }
     return;
   }
   const int nrow = ZS ? d.NZ2 : d.NY2;
   const int r0 = ZS ? a.zs : a.js, r1 = ZS ? a.ze : a.je;
   const int n2 = d.LDM * (d.NY + 3);
   const size_t sK = d.LDX, sJ = (size_t)d.LDX * d.NZ2;
-  const size_t sA = ZS ? sK : sJ;
-  const size_t sX = ZS ? sJ : sK;
-  const float *nut = a.nutf;
-  const double *R = a.R, *po = a.phi_old, *ps = a.phs;
-  const double *px = ZS ? ps : po;
+  const size_t sA = ZS ? sK : sJ, sX = ZS ? sJ : sK;
   float2 *gout = reinterpret_cast<float2 *>(a.out);
   float2 *sb = reinterpret_cast<float2 *>(a.scr_b), *su = reinterpret_cast<float2 *>(a.scr_u);
-  const size_t c0 = ZS ? d.ip(i, 0, line) : d.ip(i, line, 0);
+  const size_t c0 = (ZS ? d.ip(0, 0, line) : d.ip(0, line, 0)) + (on ? i : 0);
   const int m0 = ZS ? line * d.LDM : line, mstep = ZS ? 1 : d.LDM;
-  // chunked along y only (as in k_adi_seq)
-  constexpr int CH = ZS ? 1 : kLesChunk, CB = ZS ? 1 : kAdiChunk;
-  FF rBp(1.0f, 0.0f), gp(0.0f, 0.0f), Up(0.0f, 0.0f);
-  for (int rc = 0; rc < nrow; rc += CH) {
-    FF Lv[CH], Dv[CH], Uv[CH], Vv[CH];
+
+  // rows r, r+1 into their ring slots (one warp; every address is inside the
+  // fields: rows clamped to the line, lines to the swept ones)
+  auto build2 = [&](int r, float4 (*dst)[2][32]) {
+    const float *nut = a.nutf;
+    // lanes 0..21 fetch the two rows' eleven weights
+    const int wr = min(r + lane / 11, nrow - 1), wp = lane % 11;
+    float2 wv = make_float2(0.f, 0.f);
+    if (lane < 22 && wr >= r0 && wr <= r1) wv = a.ftab[(size_t)wp * n2 + m0 + wr * mstep];
+    float nu[4], nxp[2], nxm[2], sv[2];
+    FF f0[2], fp[2], fm[2];
 #pragma unroll
-    for (int u = 0; u < CH; ++u) {
-      const int r = rc + u;
-      const size_t c = c0 + (size_t)r * sA;
-      FF L(0.0f, 0.0f), D(1.0f, 0.0f), U(0.0f, 0.0f), V(0.0f, 0.0f);
-      if (r >= r0 && r <= r1) {
-        const float2 *t = a.ftab + (m0 + r * mstep);
-        const float nu0 = nut[c], nap = nut[c + sA], nam = nut[c - sA], nxp = nut[c + sX], nxm = nut[c - sX];
-        const FF f0(px[c]), fxp(px[c + sX]), fxm(px[c - sX]);
-        const FF rr = SF ? FF(a.Sf[c], 0.0f) : FF(R[c]);
-        FF v = FF(0.5f * rr.hi, 0.5f * rr.lo);
-        if (!ZS) {
-          v = v + ff2(t[0]) * f0 + ff2(t[n2]) * fxp + ff2(t[2 * n2]) * fxm;
-        } else if (SF) {
-          v = v + ff2(t[0]) * f0 + ff2(t[n2]) * fxp + ff2(t[2 * n2]) * fxm;
-        } else {
-          const FF p0(po[c]);
-          v = v + ff2(t[3 * n2]) * p0 + ff2(t[0]) * f0 + ff2(t[n2]) * fxp + ff2(t[2 * n2]) * fxm;
-        }
-        const FF tp = ff2(t[9 * n2]) * (ff1(nxp) + ff1(nu0)), tm = ff2(t[10 * n2]) * (ff1(nu0) + ff1(nxm));
-        V = v + tp * (fxp - f0) - tm * (f0 - fxm);
-        const FF slo = ff1(nu0) + ff1(nam), sup = ff1(nu0) + ff1(nap);
-        const FF ml = ff2(t[7 * n2]), mu = ff2(t[8 * n2]);
-        L = ff2(t[4 * n2]) - ml * slo;
-        U = ff2(t[5 * n2]) - mu * sup;
-        D = ff2(t[6 * n2]) + mu * sup + ml * slo;
-      }
-      if (r < nrow)
-        for (int b = 0; b < a.bc.n; ++b) {
-          const BcRow &br = a.bc.r[b];
-          if (br.row != r) continue;
-          L = FF(br.l);
-          D = FF(br.dg);
-          U = FF(br.u);
-          if (br.kind == 0) V = FF(br.val);
-          else if (br.kind == 1) V = FF(ZS ? ps[d.ip(i, br.src, line)] : po[d.ip(i, line, br.src)]);
-          else V = FF(br.val * a.bcw[br.src + line]);
-        }
-      Lv[u] = L;
-      Dv[u] = D;
-      Uv[u] = U;
-      Vv[u] = V;
-    }
+    for (int u = 0; u < 4; ++u) nu[u] = nut[c0 + (size_t)min(max(r - 1 + u, 0), nrow - 1) * sA];
+    double d0[2], dp[2], dm[2];
 #pragma unroll
-    for (int u = 0; u < CH; ++u) {
-      const int r = rc + u;
-      if (r >= nrow) break;
-      const size_t c = c0 + (size_t)r * sA;
-      FF B, g;
-      if (r == 0) {
-        B = Dv[u];
-        g = Vv[u];
+    for (int u = 0; u < 2; ++u) {
+      const size_t c = c0 + (size_t)min(r + u, nrow - 1) * sA;
+      nxp[u] = nut[c + sX];
+      nxm[u] = nut[c - sX];
+      sv[u] = a.Sf[c];
+      if (ZS) {
+        f0[u] = ff2(ps[c]);
+        fp[u] = ff2(ps[c + sX]);
+        fm[u] = ff2(ps[c - sX]);
       } else {
-        const FF am = -(Lv[u] * rBp);
-        B = Dv[u] + am * Up;
-        g = Vv[u] + am * gp;
+        d0[u] = po[c];
+        dp[u] = po[c + sX];
+        dm[u] = po[c - sX];
       }
-      const FF rB = ff_rcp(B);
-      gout[c] = make_float2(g.hi, g.lo);
-      sb[c] = make_float2(rB.hi, rB.lo);
-      su[c] = make_float2(Uv[u].hi, Uv[u].lo);
-      rBp = rB;
-      gp = g;
-      Up = Uv[u];
     }
+    __syncwarp();
+    if (lane < 22) wts[warp - 1][lane / 11][wp] = wv;
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int rr = r + u;
+      if (rr >= nrow) break;
+      FF L(0.0f, 0.0f), D(1.0f, 0.0f), U(0.0f, 0.0f), V(0.0f, 0.0f);
+      if (rr >= r0 && rr <= r1) {
+        const float2 *t = wts[warp - 1][u];
+        if (!ZS) {
+          f0[u] = FF(d0[u]);
+          fp[u] = FF(dp[u]);
+          fm[u] = FF(dm[u]);
+        }
+        const float nu0 = nu[u + 1];
+        const FF v = FF(0.5f * sv[u], 0.5f * 0.0f) + ff2(t[0]) * f0[u] + ff2(t[1]) * fp[u] + ff2(t[2]) * fm[u];
+        const FF tp = ff2(t[9]) * (ff1(nxp[u]) + ff1(nu0)), tm = ff2(t[10]) * (ff1(nu0) + ff1(nxm[u]));
+        V = v + tp * (fp[u] - f0[u]) - tm * (f0[u] - fm[u]);
+        const FF slo = ff1(nu0) + ff1(nu[u]), sup = ff1(nu0) + ff1(nu[u + 2]);
+        const FF ml = ff2(t[7]), mu = ff2(t[8]);
+        L = ff2(t[4]) - ml * slo;
+        U = ff2(t[5]) - mu * sup;
+        D = ff2(t[6]) + mu * sup + ml * slo;
+      }
+      for (int b = 0; b < a.bc.n; ++b) {
+        const BcRow &br = a.bc.r[b];
+        if (br.row != rr) continue;
+        L = FF(br.l);
+        D = FF(br.dg);
+        U = FF(br.u);
+        if (br.kind == 0) {
+          V = FF(br.val);
+        } else if (br.kind == 1) {
+          const size_t q = c0 + (size_t)br.src * sA;
+          V = ZS ? ff2(ps[q]) : FF(po[q]);
+        } else {
+          V = FF(br.val * a.bcw[br.src + line]);
+        }
+      }
+      dst[u][0][lane] = make_float4(L.hi, L.lo, D.hi, D.lo);
+      dst[u][1][lane] = make_float4(U.hi, U.lo, V.hi, V.lo);
+    }
+  };
+  auto build = [&](int t) {
+    for (int o = 2 * (warp - 1); o < kLesRows; o += 2 * (kLesWarps - 1)) {
+      const int r = t * kLesRows + o;
+      if (r < nrow) build2(r, &ring[t & 1][o]);
+    }
+  };
+
+  const int nch = (nrow + kLesRows - 1) / kLesRows;
+  if (warp > 0) build(0);
+  __syncthreads();
+  FF rBp(1.0f, 0.0f), gp(0.0f, 0.0f), Up(0.0f, 0.0f);
+  for (int t = 0; t < nch; ++t) {
+    if (warp > 0) {
+      if (t + 1 < nch) build(t + 1);
+    } else {
+      const int rt = t * kLesRows, n = min(kLesRows, nrow - rt);
+      float4 ld = ring[t & 1][0][0][lane], uv = ring[t & 1][0][1][lane];
+      for (int o = 0; o < n; ++o) {
+        const FF L(ld.x, ld.y), D(ld.z, ld.w), U(uv.x, uv.y), V(uv.z, uv.w);
+        const int on1 = min(o + 1, n - 1);
+        ld = ring[t & 1][on1][0][lane];
+        uv = ring[t & 1][on1][1][lane];
+        FF B, g;
+        if (rt + o == 0) {
+          B = D;
+          g = V;
+        } else {
+          const FF am = -(L * rBp);
+          B = D + am * Up;
+          g = V + am * gp;
+        }
+        const FF rB = ff_rcp(B);
+        if (on) {
+          const size_t c = c0 + (size_t)(rt + o) * sA;
+          gout[c] = make_float2(g.hi, g.lo);
+          sb[c] = make_float2(rB.hi, rB.lo);
+          su[c] = make_float2(U.hi, U.lo);
+        }
+        rBp = rB;
+        gp = g;
+        Up = U;
+      }
+    }
+    __syncthreads();
   }
-  FF x = gp * rBp;
-  a.out[c0 + (size_t)(nrow - 1) * sA] = (double)x;
-  for (int rc = nrow - 2; rc >= 0; rc -= CB) {
-    float2 gv[CB], uv[CB], bv[CB];
+  // back substitution: chunks from the line's end, each copied into the ring
+  // (g, u, b of a lane's row, 8 bytes each) while the one after it is solved
+  float2 *back = reinterpret_cast<float2 *>(&ring[0][0][0][0]);  // [slot][row][3][32]
+  constexpr int kSlot = kLesRows * 3 * 32;
+  auto fetch = [&](int t) {
+    const unsigned base = (unsigned)__cvta_generic_to_shared(back + (t & 1) * kSlot);
+    for (int o = warp - 1; o < kLesRows && t * kLesRows + o < nrow; o += kLesWarps - 1) {
+      const size_t c = c0 + (size_t)(t * kLesRows + o) * sA;
+      const float2 *src[3] = {gout + c, su + c, sb + c};
 #pragma unroll
-    for (int u = 0; u < CB; ++u) {
-      const int r = rc - u;
-      if (r >= 0) {
-        const size_t c = c0 + (size_t)r * sA;
-        gv[u] = gout[c];
-        uv[u] = su[c];
-        bv[u] = sb[c];
+      for (int p = 0; p < 3; ++p)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(base + (unsigned)(((o * 3 + p) * 32 + lane) * 8)),
+                     "l"(src[p])
+                     : "memory");
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+  };
+  if (warp > 0) fetch(nch - 1);
+  __syncthreads();
+  FF x(0.0f, 0.0f);
+  for (int t = nch - 1; t >= 0; --t) {
+    if (warp > 0) {
+      if (t > 0) fetch(t - 1);
+    } else {
+      const int rt = t * kLesRows, n = min(kLesRows, nrow - rt);
+      const float2 *bk = back + (t & 1) * kSlot + lane;
+      float2 g = bk[(n - 1) * 96], uu = bk[(n - 1) * 96 + 32], bb = bk[(n - 1) * 96 + 64];
+      for (int o = n - 1; o >= 0; --o) {
+        const FF G = ff2(g), U = ff2(uu), Bi = ff2(bb);
+        const int om = max(o - 1, 0);
+        g = bk[om * 96];
+        uu = bk[om * 96 + 32];
+        bb = bk[om * 96 + 64];
+        x = (rt + o == nrow - 1) ? G * Bi : (G - U * x) * Bi;
+        if (on) {
+          const size_t c = c0 + (size_t)(rt + o) * sA;
+          if (ZS) {
+            a.out[c] = (double)x;
+          } else {
+            const FF y = ff_round53(x);
+            gout[c] = make_float2(y.hi, y.lo);
+          }
+        }
       }
     }
-#pragma unroll
-    for (int u = 0; u < CB; ++u) {
-      const int r = rc - u;
-      if (r >= 0) {
-        x = (ff2(gv[u]) - ff2(uv[u]) * x) * ff2(bv[u]);
-        a.out[c0 + (size_t)r * sA] = (double)x;
-      }
-    }
+    __syncthreads();
   }
 }
 
@@ -1750,8 +1860,9 @@ void launch_adi(Ctx &c, int field, int rk) {
       k_adi_les_tab<true><<<tg, 64, 0, c.stream>>>(d, c.m, c.m.g11, l11, l22, coef, h, c.adi_les_tab + 7 * n2);
       after_launch(c);
     }
-    // the mixed-precision method (FP32 LES kernels) eliminates in float-float
-    const bool ff = c.les.lowp;
+    // the mixed-precision method (FP32 LES kernels, and the FP32 increment S
+    // with it) eliminates in float-float
+    const bool ff = c.les.lowp && a.Sf;
     if (ff) {
       if (!c.adi_ff_tab) {
         EK_CUDA(cudaMalloc(&c.adi_ff_tab, sizeof(float2) * 22 * n2));
@@ -1769,11 +1880,10 @@ void launch_adi(Ctx &c, int field, int rk) {
     a.ltab = c.adi_les_tab;
     a.ftab = c.adi_ff_tab;
     {
-      dim3 grid((d.NX + 127) / 128, a.ze - a.zs + 1);
+      dim3 grid((d.NX + 127) / 128, a.ze - a.zs + 1), tiles((d.NX + 31) / 32, a.ze - a.zs + 1);
       // algorithmic: read R, the field and NU_T, write the result
       KScope ks(c, KC_ADI_Y, 32.0 * d.NX * d.NY2 * (a.ze - a.zs + 1));
-      if (ff && a.Sf) k_adi_les_ff<false, true><<<grid, 128, 0, c.stream>>>(a);
-      else if (ff) k_adi_les_ff<false, false><<<grid, 128, 0, c.stream>>>(a);
+      if (ff) k_adi_les_tile<false><<<tiles, 32 * kLesWarps, 0, c.stream>>>(a);
       else if (a.Sf) k_adi_les<false, true><<<grid, 128, 0, c.stream>>>(a);
       else k_adi_les<false, false><<<grid, 128, 0, c.stream>>>(a);
       after_launch(c);
@@ -1784,11 +1894,10 @@ void launch_adi(Ctx &c, int field, int rk) {
     a.ltab = c.adi_les_tab + 7 * n2;
     a.ftab = c.adi_ff_tab ? c.adi_ff_tab + 11 * n2 : nullptr;
     {
-      dim3 grid((d.NX + 127) / 128, d.NY2);
+      dim3 grid((d.NX + 127) / 128, d.NY2), tiles((d.NX + 31) / 32, d.NY2);
       // read R, the old field, the y-sweep result and NU_T, write the result
       KScope ks(c, KC_ADI_Z, 40.0 * d.NX * d.NZ2 * (a.je - a.js + 1));
-      if (ff && a.Sf) k_adi_les_ff<true, true><<<grid, 128, 0, c.stream>>>(a);
-      else if (ff) k_adi_les_ff<true, false><<<grid, 128, 0, c.stream>>>(a);
+      if (ff) k_adi_les_tile<true><<<tiles, 32 * kLesWarps, 0, c.stream>>>(a);
       else if (a.Sf) k_adi_les<true, true><<<grid, 128, 0, c.stream>>>(a);
       else k_adi_les<true, false><<<grid, 128, 0, c.stream>>>(a);
       after_launch(c);
