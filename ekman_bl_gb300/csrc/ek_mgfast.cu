@@ -35,7 +35,7 @@ namespace {
 struct LvF {
   int nx, ny;
   float *e, *r, *cof, *cp;  // e: (0:nx+1,0:ny+1)xP; r: nx*ny*P; cof: 11*nx*ny; cp: line-solve scratch nx*ny*P
-  const float4 *cf4;        // cof packed per point (MgLevelF::cf4), for the level residual
+  const float4 *cf4;        // cof packed per point (MgLevelF::cf4)
 };
 struct FastDev {
   int P, ngrid, orth;
@@ -706,24 +706,6 @@ constexpr int kRowWarps = 8;
 // shared memory (k_f_vtail).  One definition serves both, so a level gives
 // the same numbers in either.
 
-// residual of the correction equation at point (i, j) of a level (FP32)
-__device__ __forceinline__ void f_resid_at(const float *__restrict__ cf, const float *__restrict__ ee,
-                                           const float *__restrict__ rr, float *__restrict__ scr, int nx, int ny,
-                                           int P, int p, int i, int j, float kx2, bool orth) {
-  const size_t npt = (size_t)nx * ny;
-  const size_t si = P, sj = (size_t)(nx + 2) * P;
-  const size_t pt = (size_t)(j - 1) * nx + (i - 1);
-  const float *ep = &ee[((size_t)j * (nx + 2) + i) * P + p];
-  float s = cf[pt] * ep[si] + cf[2 * npt + pt] * ep[sj] + cf[4 * npt + pt] * ep[-(long)si] +
-            cf[6 * npt + pt] * ep[-(long)sj];
-  if (!orth)
-    s += cf[npt + pt] * ep[si + sj] + cf[3 * npt + pt] * ep[sj - si] + cf[5 * npt + pt] * ep[-(long)(si + sj)] +
-         cf[7 * npt + pt] * ep[si - sj];
-  const float c9 = ((-kx2 * cf[10 * npt + pt]) - cf[8 * npt + pt]) + cf[9 * npt + pt];
-  s += c9 * ep[0];
-  scr[((size_t)j * (nx + 2) + i) * P + p] = rr[pt * P + p] - s;
-}
-
 // full weighting (res2, mudcom.f:120-257) of the fine residual in scr to the
 // coarse rhs at (ic, jc), and e_coarse = 0 there (ghosts included: ic =
 // 0..ncx+1, jc = 0..ncy+1)
@@ -751,24 +733,26 @@ __device__ __forceinline__ void f_restrict_at(const float *__restrict__ scr, flo
        4.f * R(i, j)) * .0625f;
 }
 
-// the same residual from the packed coefficients (the same products and
-// sums, in the same order): two or three vector loads for seven or eleven
-// scalar ones
+// residual r - A e of the correction equation at one point (FP32): q0 holds
+// the couplings (i+1, j+1, i-1, j-1), q2 the diagonal ones, c9 the centre
+__device__ __forceinline__ float f_resid_val(float4 q0, float4 q2, float c9, const float *ep, size_t si, size_t sj,
+                                             float rr, bool orth) {
+  float s = q0.x * ep[si] + q0.y * ep[sj] + q0.z * ep[-(long)si] + q0.w * ep[-(long)sj];
+  if (!orth) s += q2.x * ep[si + sj] + q2.y * ep[sj - si] + q2.z * ep[-(long)(si + sj)] + q2.w * ep[si - sj];
+  s += c9 * ep[0];
+  return rr - s;
+}
+// the same from the packed coefficients, at point (i, j) of a level: two or
+// three vector loads for seven or eleven scalar ones
 __device__ __forceinline__ void f_resid_at4(const float4 *__restrict__ cf4, const float *__restrict__ ee,
                                             const float *__restrict__ rr, float *__restrict__ scr, int nx, int P,
                                             int p, int i, int j, float kx2, bool orth) {
   const size_t si = P, sj = (size_t)(nx + 2) * P;
-  const size_t pt = (size_t)(j - 1) * nx + (i - 1);
-  const float *ep = &ee[((size_t)j * (nx + 2) + i) * P + p];
+  const size_t pt = (size_t)(j - 1) * nx + (i - 1), q = ((size_t)j * (nx + 2) + i) * P + p;
   const float4 q0 = cf4[3 * pt], q1 = cf4[3 * pt + 1];
-  float s = q0.x * ep[si] + q0.y * ep[sj] + q0.z * ep[-(long)si] + q0.w * ep[-(long)sj];
-  if (!orth) {
-    const float4 q2 = cf4[3 * pt + 2];
-    s += q2.x * ep[si + sj] + q2.y * ep[sj - si] + q2.z * ep[-(long)(si + sj)] + q2.w * ep[si - sj];
-  }
+  const float4 q2 = orth ? make_float4(0.f, 0.f, 0.f, 0.f) : cf4[3 * pt + 2];
   const float c9 = ((-kx2 * q1.z) - q1.x) + q1.y;
-  s += c9 * ep[0];
-  scr[((size_t)j * (nx + 2) + i) * P + p] = rr[pt * P + p] - s;
+  scr[q] = f_resid_val(q0, q2, c9, ee + q, si, sj, rr[pt * P + p], orth);
 }
 
 // residual of the correction equation at a level (FP32) into the scratch
@@ -892,20 +876,35 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_f_prolong_y(FastDev g, int l
 // d' = (d - a d') m and x = d' - c' x, with no division on the chain.
 // In: the restricted rhs of level ltop (global); out: its correction e,
 // ghosts included (global).
-constexpr int kTailThreads = 64;
+//
+// Levels lth+1..ltop, above the Thomas ones, solve their lines as k_f_pline
+// does, the same segments, separators and operations on the block's shared
+// arrays (part_lines), so a level gives the same numbers in either; with
+// ltop = ngrid a whole cycle is one launch.
+// What bounds it: the serial chain of phases (four colours a sweep, two sweeps
+// a level), each a few hundred cycles of dependent arithmetic behind a block
+// barrier; a problem's arrays never leave its SM.  Measured, a step:
+// 64 x 65 x 65 (a cycle in the block: 163,000 cycles) 4.2 -> 2.6 ms,
+// 128 x 129 x 97 sheared 15.4 -> 11.7 ms, 256 x 193 x 129 with LES 23.5 ->
+// 22.0 ms.
+constexpr int kTailThreads = 128;
 constexpr int kTailMax = 12;
+constexpr int kTailMost = 512;  // threads of a block
 struct TailPlan {
-  int ltop, sweeps;
+  int ltop, lth, sweeps;
   int nfac;  // factor floats per problem: (c', m) of the y-lines and of the x-lines, every level
   int fac0, scr, total;  // shared-memory offsets (floats): factor block, transfer scratch; total floats
   int nx[kTailMax], ny[kTailMax];
   int e[kTailMax], r[kTailMax];  // shared-memory offsets of e and r of level l + 1
   int f[kTailMax];               // offset of level l + 1's y-line factors in the factor block (x-lines follow)
+  int c[kTailMax];               // offset of its coefficients: Thomas levels the lines' lower diagonals (y, x);
+                                 // others the planes c1 c3 c5 c7 b (and c2 c4 c6 c8 unless orthogonal)
 };
 
-TailPlan make_tail_plan(const MgPlan &PL, int ltop) {
+TailPlan make_tail_plan(const MgPlan &PL, int ltop, int lth) {
   TailPlan t{};
   t.ltop = ltop;
+  t.lth = lth;
   t.sweeps = std::max(8, (PL.lv[0].nx + PL.lv[0].ny) / 2);
   int off = 0, fo = 0;
   for (int l = 0; l < ltop; ++l) {
@@ -917,14 +916,21 @@ TailPlan make_tail_plan(const MgPlan &PL, int ltop) {
     t.r[l] = off;
     off += nx * ny;
     t.f[l] = fo;
-    fo += 4 * nx * ny;
+    if (l < lth) fo += 4 * nx * ny;
   }
   t.scr = off;
   off += (t.nx[ltop - 1] + 2) * (t.ny[ltop - 1] + 2);
   off = (off + 3) & ~3;  // the factor block is copied as float4
   t.fac0 = off;
   t.nfac = fo;
-  t.total = off + fo;
+  off += fo;
+  for (int l = 0; l < ltop; ++l) {
+    t.c[l] = off;
+    off += ((l < lth) ? 2 : PL.orth ? 5 : 9) * t.nx[l] * t.ny[l];
+    off = (off + 3) & ~3;
+  }
+  // tail_chain loads whole chunks of a Thomas line's rows
+  t.total = off + kChunk * (t.nx[std::max(lth, 1) - 1] + 2);
   return t;
 }
 
@@ -933,7 +939,8 @@ struct TailLv {
   int nx, ny;
   float *e, *r;
   const float2 *fy, *fx;  // (c', m) per point, point (i, j) at (j-1) nx + (i-1)
-  const float *cof;
+  const float4 *cf4;      // packed coefficients (MgLevelF::cf4), global
+  float *c;               // staged coefficients (TailPlan::c)
 };
 __device__ __forceinline__ TailLv tail_level_at(const TailPlan &t, const FastDev &g, float *sm, int l) {
   TailLv L;
@@ -943,115 +950,423 @@ __device__ __forceinline__ TailLv tail_level_at(const TailPlan &t, const FastDev
   L.r = sm + t.r[l];
   L.fy = reinterpret_cast<const float2 *>(sm + t.fac0 + t.f[l]);
   L.fx = L.fy + (size_t)L.nx * L.ny;
-  L.cof = g.lv[l].cof;
+  L.cf4 = g.lv[l].cf4;
+  L.c = sm + t.c[l];
   return L;
 }
 
-// y-line at column i with precomputed factors (the rows of yline_solve)
-__device__ __forceinline__ void tail_yline(const TailLv &L, int i, bool orth) {
-  const int nx = L.nx, ny = L.ny, npt = nx * ny, sj = nx + 2;
-  const float *__restrict__ cf = L.cof;
-  const float *__restrict__ r = L.r;
-  const float2 *__restrict__ fy = L.fy;
+// A Thomas line's two recurrences by one thread, the rows of yline_solve and
+// xline_solve: the n right-hand sides at b[k st], replaced by the solution.
+// kChunk rows' values are loaded ahead of the recurrence (past the line's end
+// too: TailPlan pads the block's arrays for that).  gh, gh2: offsets of the
+// ghosts a y-line feeds (0: none).
+__device__ __forceinline__ void tail_chain(float *b, int st, const float *a, const float2 *f, int cst, int n, int gh,
+                                           int gh2) {
+  float prev = 0.f;
+  for (int k0 = 0; k0 < n; k0 += kChunk) {
+    float dv[kChunk], av[kChunk], mv[kChunk];
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      dv[u] = b[u * st];
+      av[u] = a[u * cst];
+      mv[u] = f[u * cst].y;
+    }
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      prev = (k0 + u < n) ? (dv[u] - av[u] * prev) * mv[u] : prev;
+      dv[u] = prev;
+    }
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u)
+      if (k0 + u < n) b[u * st] = dv[u];
+    b += kChunk * st;
+    a += kChunk * cst;
+    f += kChunk * cst;
+  }
+  float x = 0.f;
+  for (int k0 = (n - 1) / kChunk * kChunk; k0 >= 0; k0 -= kChunk) {
+    float dv[kChunk], cv[kChunk];
+    b -= kChunk * st;
+    f -= kChunk * cst;
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      dv[u] = b[u * st];
+      cv[u] = f[u * cst].x;
+    }
+#pragma unroll
+    for (int u = kChunk - 1; u >= 0; --u) {
+      x = (k0 + u < n) ? dv[u] - cv[u] * x : x;
+      dv[u] = x;
+    }
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u)
+      if (k0 + u < n) b[u * st] = dv[u];
+    if (gh | gh2)
+#pragma unroll
+      for (int u = 0; u < kChunk; ++u)
+        if (k0 + u < n) {
+          if (gh) b[u * st + gh] = dv[u];
+          if (gh2) b[u * st + gh2] = dv[u];
+        }
+  }
+}
+
+// `sweeps` alternating-direction zebra sweeps of a Thomas level by the first
+// nt threads of the block (a multiple of 32; bar: the named barrier they
+// share), in the order of the per-level relax.  A colour goes in two parts:
+// every point's right-hand side, one thread a point, into the point's own
+// place in e (a line reads only the other colour's lines), then each line's
+// recurrences.  A thread keeps its point's coefficients and right-hand side
+// over all phases (levels of more points than threads load them again).
+__device__ __forceinline__ void tail_relax(const TailLv &L, int nt, int sweeps, bool orth, bool post) {
+  const int nx = L.nx, ny = L.ny, sj = nx + 2, npt = nx * ny, tid = threadIdx.x;
+  if (tid >= nt) return;
+  auto sync = [&]() { asm volatile("bar.sync 1, %0;\n" ::"r"(nt) : "memory"); };
   float *__restrict__ e = L.e;
-  float dprev = 0.f;
-  for (int j0 = 1; j0 <= ny; j0 += kChunk) {
-    float dv[kChunk], av[kChunk], mv[kChunk];
-#pragma unroll
-    for (int u = 0; u < kChunk; ++u) {
-      const int j = j0 + u;
-      if (j > ny) break;
-      const int pt = (j - 1) * nx + (i - 1), q = j * sj + i;
-      float d = r[pt] - cf[pt] * e[q + 1] - cf[4 * npt + pt] * e[q - 1];
-      if (orth == false)
-        d = d - cf[npt + pt] * e[q + 1 + sj] - cf[3 * npt + pt] * e[q + sj - 1] - cf[5 * npt + pt] * e[q - 1 - sj] -
-            cf[7 * npt + pt] * e[q + 1 - sj];
-      dv[u] = d;
-      av[u] = cf[6 * npt + pt];
-      mv[u] = fy[pt].y;
+  struct Pt {
+    int i, j, q;
+    float r;
+    float4 k, k2;
+  };
+  auto point = [&](int v) {
+    Pt t;
+    t.j = 1 + v / nx;
+    t.i = 1 + v - (t.j - 1) * nx;
+    t.q = t.j * sj + t.i;
+    t.r = L.r[v];
+    t.k = L.cf4[3 * v];
+    t.k2 = orth ? t.k : L.cf4[3 * v + 2];
+    return t;
+  };
+  const Pt mine = point(min(tid, npt - 1));
+  auto ypoint = [&](const Pt &t) {
+    float d = t.r - t.k.x * e[t.q + 1] - t.k.z * e[t.q - 1];
+    if (orth == false)
+      d = d - t.k2.x * e[t.q + 1 + sj] - t.k2.y * e[t.q + sj - 1] - t.k2.z * e[t.q - 1 - sj] - t.k2.w * e[t.q + 1 - sj];
+    e[t.q] = d;
+  };
+  auto xpoint = [&](const Pt &t) {
+    float d = t.r - t.k.y * e[t.q + sj] - t.k.w * e[t.q - sj];
+    if (orth == false)
+      d = d - t.k2.x * e[t.q + 1 + sj] - t.k2.y * e[t.q + sj - 1] - t.k2.z * e[t.q - 1 - sj] - t.k2.w * e[t.q + 1 - sj];
+    if (t.i == 1) d -= t.k.z * e[t.j * sj];
+    if (t.i == nx) d -= t.k.x * e[t.j * sj + nx + 1];
+    e[t.q] = d;
+  };
+  for (int sw = 0; sw < sweeps; ++sw) {
+    for (int k = 0; k < 2; ++k) {
+      const int col = post ? 2 - k : 1 + k;
+      // line_phases, without its array: an even nx ends with i = 1 or nx alone
+      const bool even = nx % 2 == 0;
+      for (int q = 0; q < (even ? 2 : 1); ++q) {
+        const int i0 = (q == 1) ? (col == 1 ? 1 : nx) : (even && col == 1) ? 3 : col;
+        const int ncol = (q == 1) ? 1 : even ? nx / 2 - 1 : (col == 1) ? (nx + 1) / 2 : (nx - 1) / 2;
+        auto in = [&](int i) { return i >= i0 && i < i0 + 2 * ncol && ((i - i0) & 1) == 0; };
+        if (tid < npt && in(mine.i)) ypoint(mine);
+        for (int v = tid + nt; v < npt; v += nt) {
+          const Pt t = point(v);
+          if (in(t.i)) ypoint(t);
+        }
+        sync();
+        for (int c = tid; c < ncol; c += nt) {
+          const int i = i0 + 2 * c;
+          tail_chain(e + sj + i, sj, L.c + (i - 1), L.fy + (i - 1), nx, ny, (i == nx - 1) ? -i : 0, (i == 2) ? nx + 1 - i : 0);
+        }
+        sync();
+      }
     }
-#pragma unroll
-    for (int u = 0; u < kChunk; ++u) {
-      const int j = j0 + u;
-      if (j > ny) break;
-      dprev = (dv[u] - av[u] * dprev) * mv[u];
-      e[j * sj + i] = dprev;
+    for (int k = 0; k < 2; ++k) {
+      const int col = post ? 2 - k : 1 + k;
+      if (tid < npt && ((mine.j - col) & 1) == 0) xpoint(mine);
+      for (int v = tid + nt; v < npt; v += nt) {
+        const Pt t = point(v);
+        if (((t.j - col) & 1) == 0) xpoint(t);
+      }
+      sync();
+      for (int j = col + 2 * tid; j <= ny; j += 2 * nt) {
+        const int rb = (j - 1) * nx;
+        float *erow = e + j * sj;
+        tail_chain(erow + 1, 1, L.c + npt + rb, L.fx + rb, 1, nx, 0, 0);
+        erow[0] = erow[nx - 1];
+        erow[nx + 1] = erow[2];
+      }
+      sync();
     }
-  }
-  float x = 0.f;
-  for (int j = ny; j >= 1; --j) {
-    x = e[j * sj + i] - fy[(j - 1) * nx + (i - 1)].x * x;
-    e[j * sj + i] = x;
-    if (i == nx - 1) e[j * sj] = x;
-    if (i == 2) e[j * sj + nx + 1] = x;
-  }
-}
-
-// x-line at row j with precomputed factors (the rows of xline_solve)
-__device__ __forceinline__ void tail_xline(const TailLv &L, int j, bool orth) {
-  const int nx = L.nx, ny = L.ny, npt = nx * ny, sj = nx + 2;
-  const float *__restrict__ cf = L.cof;
-  const float *__restrict__ r = L.r;
-  const float2 *__restrict__ fx = L.fx;
-  float *__restrict__ erow = L.e + j * sj;
-  const float g0 = erow[0], g1 = erow[nx + 1];
-  const int rb = (j - 1) * nx;
-  float dprev = 0.f;
-  for (int i0 = 1; i0 <= nx; i0 += kChunk) {
-    float dv[kChunk], av[kChunk], mv[kChunk];
-#pragma unroll
-    for (int u = 0; u < kChunk; ++u) {
-      const int i = i0 + u;
-      if (i > nx) break;
-      const int pt = rb + (i - 1);
-      float d = r[pt] - cf[2 * npt + pt] * erow[i + sj] - cf[6 * npt + pt] * erow[i - sj];
-      if (orth == false)
-        d = d - cf[npt + pt] * erow[i + 1 + sj] - cf[3 * npt + pt] * erow[i + sj - 1] -
-            cf[5 * npt + pt] * erow[i - 1 - sj] - cf[7 * npt + pt] * erow[i + 1 - sj];
-      float a = cf[4 * npt + pt];
-      if (i == 1) { d -= a * g0; a = 0.f; }
-      if (i == nx) d -= cf[pt] * g1;
-      dv[u] = d;
-      av[u] = a;
-      mv[u] = fx[pt].y;
-    }
-#pragma unroll
-    for (int u = 0; u < kChunk; ++u) {
-      const int i = i0 + u;
-      if (i > nx) break;
-      dprev = (dv[u] - av[u] * dprev) * mv[u];
-      erow[i] = dprev;
-    }
-  }
-  float x = 0.f;
-  for (int i = nx; i >= 1; --i) {
-    x = erow[i] - fx[rb + (i - 1)].x * x;
-    erow[i] = x;
-    if (i == nx - 1) erow[0] = x;
-    if (i == 2) erow[nx + 1] = x;
   }
 }
 
-// one alternating-direction zebra sweep (the order of the per-level relax)
-__device__ __forceinline__ void tail_relax(const TailLv &L, bool orth, bool post) {
-  for (int k = 0; k < 2; ++k) {
-    const int col = post ? 2 - k : 1 + k;
-    LinePhase ph[2];
-    const int nph = line_phases(L.nx, col, ph);
-    for (int q = 0; q < nph; ++q) {
-      for (int c = threadIdx.x; c < ph[q].ncol; c += blockDim.x) tail_yline(L, ph[q].i0 + ph[q].istep * c, orth);
+// The same sweeps of a level of at most 32 points and N rows and columns (the
+// coarsest one: many sweeps of a few points) by one warp, lane = point, e in
+// registers.  A line's right-hand sides are gathered by shuffles and every
+// lane of the line runs the line's recurrences, with the coefficients of its
+// row and column in registers: no shared-memory round trip and no barrier
+// stands between the phases.  A ghost column always equals the column it
+// copies, and the rows outside the level are zero.
+template <int N>
+__device__ __forceinline__ void tail_coarse(const TailLv &L, int sweeps, bool orth) {
+  const int nx = L.nx, ny = L.ny, sj = nx + 2, npt = nx * ny;
+  const unsigned all = 0xffffffffu;
+  const int v = min((int)(threadIdx.x & 31), npt - 1);
+  const int j = v / nx, i = v - j * nx;  // from 0
+  const int vl = v - i + ((i == 0) ? nx - 2 : i - 1), vr = v - i + ((i == nx - 1) ? 1 : i + 1);
+  const bool hasn = j < ny - 1, hass = j > 0;
+  const int up = hasn ? nx : 0, dn = hass ? -nx : 0;
+  const float4 k = L.cf4[3 * v], k2 = orth ? k : L.cf4[3 * v + 2];
+  const float r = L.r[v];
+  float ay[N], my[N], cy[N], ax[N], mx[N], cx[N];
+#pragma unroll
+  for (int t = 0; t < N; ++t) {
+    const int py = min(t, ny - 1) * nx + i, px = j * nx + min(t, nx - 1);
+    ay[t] = L.c[py];
+    my[t] = L.fy[py].y;
+    cy[t] = L.fy[py].x;
+    ax[t] = L.c[npt + px];
+    mx[t] = L.fx[px].y;
+    cx[t] = L.fx[px].x;
+  }
+  float e = 0.f;
+  auto diag = [&](float d) {
+    const float a = __shfl_sync(all, e, vr + up), b = __shfl_sync(all, e, vl + up);
+    const float c = __shfl_sync(all, e, vl + dn), f = __shfl_sync(all, e, vr + dn);
+    return d - k2.x * (hasn ? a : 0.f) - k2.y * (hasn ? b : 0.f) - k2.z * (hass ? c : 0.f) - k2.w * (hass ? f : 0.f);
+  };
+  // the line's solution at this lane's place (m) from its right-hand sides
+  auto chain = [&](float d, int v0, int st, int n, int m, const float *a, const float *mm, const float *c) {
+    float w[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) w[t] = __shfl_sync(all, d, v0 + min(t, n - 1) * st);
+    float prev = 0.f;
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      prev = (w[t] - a[t] * prev) * mm[t];
+      w[t] = prev;
+    }
+    float x = 0.f, mine = 0.f;
+#pragma unroll
+    for (int t = N - 1; t >= 0; --t) {
+      x = (t < n) ? w[t] - c[t] * x : 0.f;
+      mine = (t == m) ? x : mine;
+    }
+    return mine;
+  };
+  const bool even = nx % 2 == 0;
+  for (int sw = 0; sw < sweeps; ++sw) {
+    for (int q = 0; q < (even ? 4 : 2); ++q) {
+      // the phases of line_phases: columns 1 3 5 .. and 2 4 .. (from 1); an
+      // even nx: 3 5 .., 1, 2 4 .. nx-2, nx
+      bool in;
+      if (!even) in = (i & 1) == q;
+      else if (q == 0) in = (i & 1) == 0 && i > 0;
+      else if (q == 1) in = i == 0;
+      else if (q == 2) in = (i & 1) == 1 && i < nx - 1;
+      else in = i == nx - 1;
+      const float er = __shfl_sync(all, e, vr), el = __shfl_sync(all, e, vl);
+      float d = r - k.x * er - k.z * el;
+      if (orth == false) d = diag(d);
+      const float x = chain(d, i, nx, ny, j, ay, my, cy);
+      e = in ? x : e;
+    }
+    for (int col = 0; col < 2; ++col) {
+      const float en = __shfl_sync(all, e, v + up), es = __shfl_sync(all, e, v + dn);
+      const float g0 = __shfl_sync(all, e, v - i + nx - 2), g1 = __shfl_sync(all, e, v - i + 1);
+      float d = r - k.y * (hasn ? en : 0.f) - k.w * (hass ? es : 0.f);
+      if (orth == false) d = diag(d);
+      if (i == 0) d -= k.z * g0;
+      if (i == nx - 1) d -= k.x * g1;
+      const float x = chain(d, j * nx, 1, nx, i, ax, mx, cx);
+      e = ((j & 1) == col) ? x : e;
+    }
+  }
+  float *row = L.e + (j + 1) * sj;
+  row[i + 1] = e;
+  if (i == nx - 2) row[0] = e;
+  if (i == 1) row[nx + 1] = e;
+}
+
+// The lines l0, l0 + lstep, ... (nline of them) of one colour by the whole
+// block, k_f_pline's partitioned solve operation for operation: thread (s, li)
+// owns segment s of line li, G lines at a time, sh the scratch of SH_N arrays
+// of K x G.  The level's coefficients and the problem's diagonal are staged in
+// shared memory: read from L2, a colour's 110 KB (65 x 65) at an SM's share of
+// the L2 bandwidth took longer than the solve.
+template <bool XL, bool ORTH>
+__device__ __forceinline__ void part_lines(const TailLv &L, float *sh, int l0, int lstep, int nline) {
+  constexpr int SEG = 8;
+  const int nx = L.nx, ny = L.ny, n = XL ? nx : ny, sj = nx + 2, npt = nx * ny;
+  const int K = max(1, (n + SEG + 1) / (SEG + 1));
+  const int mb = (n - K + 1) / K, me = (n - K + 1) - mb * K;
+  const int G = min((int)blockDim.x / K, nline);
+  const int s0 = (int)threadIdx.x / G, li = (int)threadIdx.x - s0 * G;
+  const int s = min(s0, K - 1);
+  auto S = [&](int arr, int seg) -> float & { return sh[(arr * K + seg) * G + li]; };
+  const int m = mb + (s < me ? 1 : 0);
+  const int lo = 1 + s * (mb + 1) + min(s, me);
+  const int nsep = K - 1;
+  for (int g0 = 0; g0 < nline; g0 += G) {
+    const bool act = s0 < K && g0 + li < nline;
+    const int line = act ? l0 + lstep * (g0 + li) : l0;
+    auto row = [&](int k, float &a, float &b, float &c, float &d) {
+      const int i = XL ? k : line, j = XL ? line : k;
+      const int pt = (j - 1) * nx + (i - 1);
+      const float *ep = L.e + (j * sj + i);
+      const float *cp = L.c + pt;
+      b = cp[4 * npt];
+      float dd = L.r[pt];
+      if (XL) {
+        a = cp[2 * npt];
+        c = cp[0];
+        dd = dd - cp[npt] * ep[sj] - cp[3 * npt] * ep[-sj];
+      } else {
+        a = cp[3 * npt];
+        c = cp[npt];
+        dd = dd - cp[0] * ep[1] - cp[2 * npt] * ep[-1];
+      }
+      if (!ORTH)
+        dd = dd - cp[5 * npt] * ep[1 + sj] - cp[6 * npt] * ep[sj - 1] - cp[7 * npt] * ep[-(1 + sj)] -
+             cp[8 * npt] * ep[-(sj - 1)];
+      d = dd;
+    };
+    auto store = [&](int k, float x) {
+      const int i = XL ? k : line, j = XL ? line : k;
+      float *erow = L.e + j * sj;
+      erow[i] = x;
+      if (i == nx - 1) erow[0] = x;
+      if (i == 2) erow[nx + 1] = x;
+    };
+    float av[SEG], bv[SEG], cv[SEG], dv[SEG];
+    // (threads beyond the group's lines and segments only keep the barriers)
+    if (act) {
+#pragma unroll
+      for (int u = 0; u < SEG; ++u) row(lo + min(u, m - 1), av[u], bv[u], cv[u], dv[u]);
+      if (XL) {
+        const float *erow = L.e + line * sj;
+        if (s == 0) {
+          dv[0] -= av[0] * erow[0];
+          av[0] = 0.f;
+        }
+        if (s == K - 1) {
+          const float gh = erow[nx + 1];
+#pragma unroll
+          for (int u = 0; u < SEG; ++u) {
+            const bool hit = (u == m - 1);
+            dv[u] = hit ? dv[u] - cv[u] * gh : dv[u];
+            cv[u] = hit ? 0.f : cv[u];
+          }
+        }
+      }
+      float yl = 0.f, vl = 0.f, wl = 0.f;
+      {
+        float bprev = 0.f, dprev = 0.f, gprev = 1.f;
+#pragma unroll
+        for (int u = 0; u < SEG; ++u) {
+          const float inv = __fdividef(1.f, bv[u] - av[u] * bprev);
+          bprev = cv[u] * inv;
+          dprev = (dv[u] - av[u] * dprev) * inv;
+          gprev = -av[u] * gprev * inv;
+          cv[u] = bprev;
+          dv[u] = dprev;
+          av[u] = gprev;
+          const bool last = (u == m - 1);
+          yl = last ? dprev : yl;
+          vl = last ? gprev : vl;
+          wl = last ? -bprev : wl;
+        }
+      }
+      float yf = yl, vf = vl, wf = wl;
+#pragma unroll
+      for (int u = SEG - 2; u >= 0; --u)
+        if (u < m - 1) {
+          yf = dv[u] - cv[u] * yf;
+          vf = av[u] - cv[u] * vf;
+          wf = -cv[u] * wf;
+        }
+      S(SH_YF, s) = yf; S(SH_VF, s) = vf; S(SH_WF, s) = wf;
+      S(SH_YL, s) = yl; S(SH_VL, s) = vl; S(SH_WL, s) = wl;
+      if (s < nsep) {
+        float a, b, c, d;
+        row(lo + m, a, b, c, d);
+        S(SH_A, s) = a; S(SH_B, s) = b; S(SH_C, s) = c; S(SH_D, s) = d;
+      }
+    }
+    __syncthreads();
+    const bool sep = act && s0 < nsep;
+    float eA = 0.f, eB = 1.f, eC = 0.f, eD = 0.f;
+    if (sep) {
+      const float a = S(SH_A, s), c = S(SH_C, s);
+      eA = (s > 0) ? a * S(SH_VL, s) : 0.f;
+      eB = S(SH_B, s) + a * S(SH_WL, s) + c * S(SH_VF, s + 1);
+      eC = (s < nsep - 1) ? c * S(SH_WF, s + 1) : 0.f;
+      eD = S(SH_D, s) - a * S(SH_YL, s) - c * S(SH_YF, s + 1);
+    }
+    // (the rows go to two sets of arrays in turn, so that a step needs one
+    // barrier: a set is written again only after the barrier behind which
+    // everyone has read the other; the first set's entries were read by their
+    // own thread alone, the second's neighbours before the first barrier)
+    int set = 0;
+    for (int d = 1; d < nsep; d <<= 1, set ^= 1) {
+      const int qA = set ? SH_YF : SH_A, qB = set ? SH_VF : SH_B, qC = set ? SH_WF : SH_C, qD = set ? SH_YL : SH_D;
+      if (sep) {
+        S(qA, s) = eA;
+        S(qB, s) = eB;
+        S(qC, s) = eC;
+        S(qD, s) = eD;
+      }
       __syncthreads();
+      if (sep) {
+        float nA = 0.f, nC = 0.f, nB = eB, nD = eD;
+        if (s - d >= 0) {
+          const float al = __fdividef(eA, S(qB, s - d));
+          nA = -al * S(qA, s - d);
+          nB -= al * S(qC, s - d);
+          nD -= al * S(qD, s - d);
+        }
+        if (s + d < nsep) {
+          const float ga = __fdividef(eC, S(qB, s + d));
+          nC = -ga * S(qC, s + d);
+          nB -= ga * S(qA, s + d);
+          nD -= ga * S(qD, s + d);
+        }
+        eA = nA;
+        eB = nB;
+        eC = nC;
+        eD = nD;
+      }
     }
-  }
-  for (int k = 0; k < 2; ++k) {
-    const int col = post ? 2 - k : 1 + k;
-    const int nrow = (L.ny >= col) ? (L.ny - col) / 2 + 1 : 0;
-    for (int c = threadIdx.x; c < nrow; c += blockDim.x) tail_xline(L, col + 2 * c, orth);
+    if (sep) S(SH_S, s) = __fdividef(eD, eB);
+    __syncthreads();
+    if (act) {
+      const float X0 = (s > 0) ? S(SH_S, s - 1) : 0.f;
+      const float X1 = (s < nsep) ? S(SH_S, s) : 0.f;
+      float x = 0.f;
+#pragma unroll
+      for (int u = SEG - 1; u >= 0; --u)
+        if (u < m) {
+          x = dv[u] + av[u] * X0 - cv[u] * ((u == m - 1) ? X1 : x);
+          store(lo + u, x);
+        }
+      if (s < nsep) store(lo + m, X1);
+    }
     __syncthreads();
   }
 }
 
-// Thomas factors of every line of the levels 1..ltop, per problem (one block
+// part_lines' zebra sweep at one level (tail_relax's order)
+template <bool ORTH>
+__device__ __forceinline__ void part_relax(const TailLv &L, float *sh, bool post) {
+  for (int k = 0; k < 2; ++k) {
+    const int col = post ? 2 - k : 1 + k;
+    LinePhase ph[2];
+    const int nph = line_phases(L.nx, col, ph);
+    for (int q = 0; q < nph; ++q)
+      if (ph[q].ncol > 0) part_lines<false, ORTH>(L, sh, ph[q].i0, ph[q].istep, ph[q].ncol);
+  }
+  for (int k = 0; k < 2; ++k) {
+    const int col = post ? 2 - k : 1 + k;
+    part_lines<true, ORTH>(L, sh, col, 2, (L.ny - col) / 2 + 1);
+  }
+}
+
+// Thomas factors of every line of the levels 1..lth, per problem (one block
 // per problem), into fac[p * nfac ...] in the shared-memory layout of the
 // factor block; the same m and c' as yline_solve / xline_solve compute
 __global__ void __launch_bounds__(kTailThreads) k_f_tail_factors(FastDev g, TailPlan t, float *fac) {
@@ -1059,96 +1374,161 @@ __global__ void __launch_bounds__(kTailThreads) k_f_tail_factors(FastDev g, Tail
   if (p >= g.P) return;
   const float kx2 = (float)g.kx2[p];
   float *fb = fac + (size_t)p * t.nfac;
-  for (int l = 0; l < t.ltop; ++l) {
+  for (int l = 0; l < t.lth; ++l) {
     const int nx = t.nx[l], ny = t.ny[l], npt = nx * ny;
-    const float *__restrict__ cf = g.lv[l].cof;
+    const float4 *__restrict__ cf4 = g.lv[l].cf4;
     float2 *fy = reinterpret_cast<float2 *>(fb + t.f[l]);
     float2 *fx = fy + npt;
-    for (int i = 1 + threadIdx.x; i <= nx; i += blockDim.x) {
+    // the y-lines on the first threads, the x-lines on the next; a chunk's
+    // coefficients are loaded before the divisions run through it
+    for (int t0 = threadIdx.x; t0 < nx + ny; t0 += blockDim.x) {
+      const bool yl = t0 < nx;
+      const int n = yl ? ny : nx, step = yl ? nx : 1, pt0 = yl ? t0 : (t0 - nx) * nx;
+      float2 *f = yl ? fy : fx;
       float cprev = 0.f;
-      for (int j = 1; j <= ny; ++j) {
-        const int pt = (j - 1) * nx + (i - 1);
-        const float b = ((-kx2 * cf[10 * npt + pt]) - cf[8 * npt + pt]) + cf[9 * npt + pt];
-        const float m = 1.f / (b - cf[6 * npt + pt] * cprev);
-        cprev = cf[2 * npt + pt] * m;
-        fy[pt] = make_float2(cprev, m);
-      }
-    }
-    for (int j = 1 + threadIdx.x; j <= ny; j += blockDim.x) {
-      float cprev = 0.f;
-      for (int i = 1; i <= nx; ++i) {
-        const int pt = (j - 1) * nx + (i - 1);
-        const float b = ((-kx2 * cf[10 * npt + pt]) - cf[8 * npt + pt]) + cf[9 * npt + pt];
-        const float a = (i == 1) ? 0.f : cf[4 * npt + pt];
-        const float c = (i == nx) ? 0.f : cf[pt];
-        const float m = 1.f / (b - a * cprev);
-        cprev = c * m;
-        fx[pt] = make_float2(cprev, m);
+      for (int k0 = 0; k0 < n; k0 += kChunk) {
+        float bv[kChunk], av[kChunk], cv[kChunk];
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+          const int k = min(k0 + u, n - 1), pt = pt0 + k * step;
+          const float4 q0 = cf4[3 * pt], q1 = cf4[3 * pt + 1];
+          bv[u] = ((-kx2 * q1.z) - q1.x) + q1.y;
+          av[u] = yl ? q0.w : (k == 0) ? 0.f : q0.z;
+          cv[u] = yl ? q0.y : (k == n - 1) ? 0.f : q0.x;
+        }
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u)
+          if (k0 + u < n) {
+            const float m = 1.f / (bv[u] - av[u] * cprev);
+            cprev = cv[u] * m;
+            f[pt0 + (k0 + u) * step] = make_float2(cprev, m);
+          }
       }
     }
   }
 }
 
-__global__ void __launch_bounds__(kTailThreads) k_f_vtail(FastDev g, TailPlan t, const float *fac) {
+template <bool ORTH>
+__global__ void __launch_bounds__(kTailMost) k_f_vtail(FastDev g, TailPlan t, const float *fac) {
   if (*g.alldone) return;
   const int p = (int)blockIdx.x;
   if (p >= g.P || g.done[p]) return;
   extern __shared__ __align__(16) float tsh[];
   const int P = g.P;
   const float kx2 = (float)g.kx2[p];
-  const bool orth = g.orth != 0;
   const int ltop = t.ltop;
   float *const scr = tsh + t.scr;
   {
-    // this problem's factors (contiguous), the rhs of level ltop, e = 0
-    const float4 *src = reinterpret_cast<const float4 *>(fac + (size_t)p * t.nfac);
-    float4 *dst = reinterpret_cast<float4 *>(tsh + t.fac0);
-    for (int v = threadIdx.x; v < t.nfac / 4; v += blockDim.x) dst[v] = src[v];
+    // this problem's factors (contiguous), the rhs of level ltop, e = 0 and the
+    // coefficients, as asynchronous copies where they move unchanged
+    auto cp16 = [](float *dst, const void *src) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                   : "memory");
+    };
+    auto cp4 = [](float *dst, const void *src) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                   : "memory");
+    };
+    const float *src = fac + (size_t)p * t.nfac;
+    for (int v = threadIdx.x; v < t.nfac / 4; v += blockDim.x) cp16(tsh + t.fac0 + 4 * v, src + 4 * v);
     const TailLv T = tail_level_at(t, g, tsh, ltop - 1);
     const LvF &G = g.lv[ltop - 1];
     const int ne = (T.nx + 2) * (T.ny + 2), nr = T.nx * T.ny;
+    for (int v = threadIdx.x; v < nr; v += blockDim.x) cp4(T.r + v, G.r + ((size_t)v * P + p));
+    for (int l = t.lth; l < ltop; ++l) {
+      const TailLv L = tail_level_at(t, g, tsh, l);
+      const int npt = L.nx * L.ny;
+      for (int v = threadIdx.x; v < npt; v += blockDim.x) {
+        // one plane a coefficient: a line's rows and a colour's lines then
+        // read distinct banks (packed float4 rows cost the solves 20%)
+        const float *f = reinterpret_cast<const float *>(L.cf4 + 3 * v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          cp4(L.c + q * npt + v, f + q);
+          if (!ORTH) cp4(L.c + (5 + q) * npt + v, f + 8 + q);
+        }
+      }
+    }
     for (int v = threadIdx.x; v < ne; v += blockDim.x) T.e[v] = 0.f;
-    for (int v = threadIdx.x; v < nr; v += blockDim.x) T.r[v] = G.r[(size_t)v * P + p];
+    for (int l = 0; l < ltop; ++l) {
+      const TailLv L = tail_level_at(t, g, tsh, l);
+      const int npt = L.nx * L.ny;
+      if (l < t.lth) {
+        // the lower diagonals of the y-lines and of the x-lines (none at i = 1)
+        for (int v = threadIdx.x; v < npt; v += blockDim.x) {
+          const float4 q0 = L.cf4[3 * v];
+          L.c[v] = q0.w;
+          L.c[npt + v] = (v % L.nx == 0) ? 0.f : q0.z;
+        }
+      } else {
+        float *cb = L.c + 4 * npt;
+#pragma unroll 8
+        for (int v = threadIdx.x; v < npt; v += blockDim.x) {
+          const float4 q1 = L.cf4[3 * v + 1];
+          cb[v] = ((-kx2 * q1.z) - q1.x) + q1.y;
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
   }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = (int)blockDim.x >> 5;
   __syncthreads();
-  for (int l = ltop; l >= 2; --l) {
-    const TailLv F = tail_level_at(t, g, tsh, l - 1), C = tail_level_at(t, g, tsh, l - 2);
-    tail_relax(F, orth, false);
-    for (int v = threadIdx.x; v < F.nx * F.ny; v += blockDim.x)
-      f_resid_at(F.cof, F.e, F.r, scr, F.nx, F.ny, 1, 0, 1 + v % F.nx, 1 + v / F.nx, kx2, orth);
+  // down the levels ltop..2, the coarsest, and up again (one place for each
+  // operation: a second copy of the line solves costs the block its registers)
+  for (int st = 0; st < 2 * ltop - 1; ++st) {
+    const bool down = st < ltop - 1, up = st >= ltop;
+    const int l = down ? ltop - st : up ? st - ltop + 2 : 1;
+    const TailLv F = tail_level_at(t, g, tsh, l - 1), C = tail_level_at(t, g, tsh, max(l - 2, 0));
+    if (up) {
+      const int nrr = (C.ny < F.ny) ? (F.ny + 1) / 2 : F.ny;
+      for (int rr = warp; rr < nrr; rr += nw)
+        for (int i = 1 + lane; i <= F.nx; i += 32)
+          f_prolong_x_at(C.e, scr, F.nx, F.ny, C.nx, C.ny, 1, 0, i, rr);
+      __syncthreads();
+      for (int j = 1 + warp; j <= F.ny; j += nw)
+        for (int i = 1 + lane; i <= F.nx; i += 32) f_prolong_y_at(scr, F.e, F.nx, F.ny, C.ny, 1, 0, i, j);
+      __syncthreads();
+    }
+    // a Thomas level's threads: one a point, whole warps, at most the block
+    if (l == 1 && F.nx * F.ny <= 32 && max(F.nx, F.ny) <= 5) {
+      if (warp == 0) tail_coarse<5>(F, t.sweeps, ORTH);
+    } else if (l > t.lth) part_relax<ORTH>(F, scr, up);
+    else tail_relax(F, min((int)blockDim.x, (F.nx * F.ny + 31) & ~31), (l == 1) ? t.sweeps : 1, ORTH, up);
     __syncthreads();
-    for (int v = threadIdx.x; v < (C.nx + 2) * (C.ny + 2); v += blockDim.x)
-      f_restrict_at(scr, C.e, C.r, F.nx, F.ny, C.nx, C.ny, 1, 0, v % (C.nx + 2), v / (C.nx + 2));
-    __syncthreads();
-  }
-  {
-    const TailLv L = tail_level_at(t, g, tsh, 0);
-    for (int sw = 0; sw < t.sweeps; ++sw) tail_relax(L, orth, false);
-    if (kx2 == 0.f) {
+    if (l == 1 && kx2 == 0.f) {
       // singular: keep the correction at zero mean, ghosts included (the
       // sum in k_f_coarsest's order)
       __shared__ float mean;
       if (threadIdx.x == 0) {
         float m = 0.f;
-        for (int j = 1; j <= L.ny; ++j)
-          for (int i = 1; i <= L.nx; ++i) m += L.e[j * (L.nx + 2) + i];
-        mean = m / (float)(L.nx * L.ny);
+        for (int j = 1; j <= F.ny; ++j)
+          for (int i = 1; i <= F.nx; ++i) m += F.e[j * (F.nx + 2) + i];
+        mean = m / (float)(F.nx * F.ny);
       }
       __syncthreads();
-      for (int v = threadIdx.x; v < L.ny * (L.nx + 2); v += blockDim.x) L.e[(L.nx + 2) + v] -= mean;
+      for (int v = threadIdx.x; v < F.ny * (F.nx + 2); v += blockDim.x) F.e[(F.nx + 2) + v] -= mean;
       __syncthreads();
     }
-  }
-  for (int l = 2; l <= ltop; ++l) {
-    const TailLv F = tail_level_at(t, g, tsh, l - 1), C = tail_level_at(t, g, tsh, l - 2);
-    const int nrr = (C.ny < F.ny) ? (F.ny + 1) / 2 : F.ny;
-    for (int v = threadIdx.x; v < F.nx * nrr; v += blockDim.x)
-      f_prolong_x_at(C.e, scr, F.nx, F.ny, C.nx, C.ny, 1, 0, 1 + v % F.nx, v / F.nx);
-    __syncthreads();
-    for (int v = threadIdx.x; v < F.nx * F.ny; v += blockDim.x)
-      f_prolong_y_at(scr, F.e, F.nx, F.ny, C.ny, 1, 0, 1 + v % F.nx, 1 + v / F.nx);
-    __syncthreads();
-    tail_relax(F, orth, true);
+    if (down) {
+      for (int j = 1 + warp; j <= F.ny; j += nw)
+        for (int i = 1 + lane; i <= F.nx; i += 32) {
+          if (l > t.lth) {
+            const int npt = F.nx * F.ny, v = (j - 1) * F.nx + i - 1, q = j * (F.nx + 2) + i;
+            const float *cp = F.c + v;
+            const float4 q0 = make_float4(cp[0], cp[npt], cp[2 * npt], cp[3 * npt]);
+            const float4 q2 = ORTH ? q0 : make_float4(cp[5 * npt], cp[6 * npt], cp[7 * npt], cp[8 * npt]);
+            scr[q] = f_resid_val(q0, q2, cp[4 * npt], F.e + q, 1, (size_t)(F.nx + 2), F.r[v], ORTH);
+          } else {
+            f_resid_at4(F.cf4, F.e, F.r, scr, F.nx, 1, 0, i, j, kx2, ORTH);
+          }
+        }
+      __syncthreads();
+      for (int jc = warp; jc <= C.ny + 1; jc += nw)
+        for (int ic = lane; ic <= C.nx + 1; ic += 32)
+          f_restrict_at(scr, C.e, C.r, F.nx, F.ny, C.nx, C.ny, 1, 0, ic, jc);
+      __syncthreads();
+    }
   }
   {
     const TailLv T = tail_level_at(t, g, tsh, ltop - 1);
@@ -1264,20 +1644,50 @@ FastDev make_fastdev(Ctx &c, int nprob, const double *kx2_dev) {
   return g;
 }
 
-// shared memory of k_f_vtail: at most this much.  Measured on the
-// 512 x 385 x 257 workload (levels 3x4 .. 257x385): the levels up to 17 x 25
-// in the tail (17 KB) beat up to 33 x 49 (62 KB) by 0.8 ms a step -- a level
-// of ~1,600 points is cheaper as batched launches than on one block's
-// thread chain, and the smaller blocks leave L1 to the coefficients.
+// The levels of k_f_vtail whose lines go one thread each (Thomas factors): the
+// largest level below the finest whose iterates, right-hand sides and factors
+// fit kTailSmem bytes (0: none fits, k_f_coarsest).
 constexpr size_t kTailSmem = 24 * 1024;
-// the levels 1..ltop that k_f_vtail runs: the largest ltop below the finest
-// level whose arrays fit kTailSmem bytes (0: none fits, k_f_coarsest)
-int tail_level(const MgPlan &PL) {
-  int ltop = 0;
-  while (ltop + 1 < PL.ngrid && ltop + 1 <= kTailMax &&
-         make_tail_plan(PL, ltop + 1).total * sizeof(float) <= kTailSmem)
-    ++ltop;
-  return ltop;
+int thomas_levels(const MgPlan &PL) {
+  int l = 0;
+  while (l + 1 < PL.ngrid && l + 1 <= kTailMax && make_tail_plan(PL, l + 1, l + 1).c[0] * sizeof(float) <= kTailSmem)
+    ++l;
+  return l;
+}
+constexpr size_t kTailMostSmem = 220 * 1024;
+constexpr int kSMs = 152;
+size_t tail_bytes_of(const TailPlan &t) { return (size_t)t.total * sizeof(float); }
+// Threads of a k_f_vtail block (128 registers each): the whole register file
+// while every problem has an SM of its own, half of it when two blocks share
+// one.
+int tail_threads(const TailPlan &t, int nprob) {
+  if (t.ltop == t.lth) return kTailThreads;
+  return (nprob <= kSMs) ? kTailMost : kTailMost / 2;
+}
+// The levels 1..ltop that run as one k_f_vtail launch for nprob problems: the
+// largest whose arrays fit one SM's shared memory while every problem has an
+// SM of its own, half of it beyond.  With fewer problems than SMs a level's
+// batched launches leave the GPU idle between their dependent steps
+// (44 problems of 65 x 65: 12 launches a level and cycle of 5-9 us each, 27 us
+// in the block); with 342 problems a level of 65 x 97 in the block costs
+// 15.2 -> 16.2 ms a batch, and 33 x 49 gains 1% over leaving it out.  A level
+// whose line-solve layout was set by hand keeps its launches.
+bool layout_set(const MgPlan &PL, int l) {
+  for (const std::vector<int> *v : {&PL.lanes_y, &PL.lanes_x, &PL.seg_y, &PL.seg_x})
+    if (l < (int)v->size() && (*v)[l] > 0) return true;
+  return false;
+}
+int tail_level(const MgPlan &PL, int nprob) {
+  const int lth = thomas_levels(PL);
+  if (lth == 0) return 0;
+  const size_t most = (nprob <= kSMs) ? kTailMostSmem : kTailMostSmem / 2;
+  // (k_f_pline takes lines of at most 567 rows at 16 problems a block; longer
+  // ones go one thread a line, in another order of operations)
+  int top = lth;
+  while (top + 1 <= PL.ngrid && top + 1 <= kTailMax && !layout_set(PL, top + 1) && std::max(PL.lv[top].nx, PL.lv[top].ny) <= 567 &&
+         tail_bytes_of(make_tail_plan(PL, top + 1, lth)) <= most)
+    ++top;
+  return top;
 }
 
 void launch_resid_ff(const FastDev &g, bool update, unsigned pch, cudaStream_t s) {
@@ -1300,7 +1710,7 @@ unsigned nb(long n, int bs) {
 
 }  // namespace
 
-int mgfast_tail_levels(const Ctx &c) { return c.mg.ngrid > 0 ? tail_level(c.mg) : 0; }
+int mgfast_tail_levels(const Ctx &c) { return c.mg.ngrid > 0 ? thomas_levels(c.mg) : 0; }
 
 // FP32 copies of the level coefficients and the FP32 work arrays.
 void mgfast_alloc(Ctx &c, int pmax) {
@@ -1321,8 +1731,8 @@ void mgfast_alloc(Ctx &c, int pmax) {
   tot += nph * pmax;
   const size_t ff_off = tot;
   tot += 4 * nph * pmax + 2 * nf * pmax + 22 * nf + 1;
-  const int ltop = tail_level(PL);
-  const size_t nfac = ltop ? (size_t)make_tail_plan(PL, ltop).nfac * pmax : 0;
+  const int lth = thomas_levels(PL);
+  const size_t nfac = lth ? (size_t)make_tail_plan(PL, lth, lth).nfac * pmax : 0;
   tot = (tot + 3) & ~(size_t)3;  // float4 reads of each problem's factor block
   const size_t fac_off = tot;
   tot += nfac;
@@ -1377,9 +1787,10 @@ void mgfast_alloc(Ctx &c, int pmax) {
   }
   c.mgf_tailfac = nfac ? c.mgf_pool + fac_off : nullptr;
   c.mgf_tailfac_n = nfac;
-  // every context's tail fits kTailSmem, so one process-wide limit serves all
-  // (set here, never during a stream capture)
-  EK_CUDA(cudaFuncSetAttribute(k_f_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
+  // every context's tail fits kTailMostSmem, so one process-wide limit serves
+  // all (set here, never during a stream capture)
+  EK_CUDA(cudaFuncSetAttribute(k_f_vtail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailMostSmem));
+  EK_CUDA(cudaFuncSetAttribute(k_f_vtail<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailMostSmem));
   {
     // the finest coefficients split into float-float pairs
     const std::vector<double> &cf = PL.cof_host[PL.ngrid - 1];
@@ -1517,9 +1928,8 @@ int mgfast_solve(Ctx &c, int nprob, const double *kx2_dev, const double *kx2_hos
     after_launch(c);
   };
   // the levels 1..ltop run as one k_f_vtail launch
-  const int ltop = tail_level(PL);
-  const TailPlan tplan = ltop ? make_tail_plan(PL, ltop) : TailPlan{};
-  const size_t tail_bytes = ltop ? tplan.total * sizeof(float) : 0;
+  const int ltop = tail_level(PL, nprob);
+  const TailPlan tplan = ltop ? make_tail_plan(PL, ltop, thomas_levels(PL)) : TailPlan{};
   if (ltop) {
     if ((size_t)tplan.nfac * nprob > c.mgf_tailfac_n) throw CudaError("mixed solve: tail factor buffer too small");
     KScope ks(c, KC_MG_SETUP, 4.0 * nprob * tplan.nfac);
@@ -1541,7 +1951,9 @@ int mgfast_solve(Ctx &c, int nprob, const double *kx2_dev, const double *kx2_hos
       if (l == ltop) {
         // bytes: level ltop's rhs in and its correction out
         KScope ks(c, KC_MG_COARSE, 4.0 * nprob * (L.nx * L.ny + (L.nx + 2.0) * (L.ny + 2)));
-        k_f_vtail<<<(unsigned)nprob, kTailThreads, tail_bytes, s>>>(g, tplan, c.mgf_tailfac);
+        const int nt = tail_threads(tplan, nprob);
+        if (g.orth) k_f_vtail<true><<<(unsigned)nprob, nt, tail_bytes_of(tplan), s>>>(g, tplan, c.mgf_tailfac);
+        else k_f_vtail<false><<<(unsigned)nprob, nt, tail_bytes_of(tplan), s>>>(g, tplan, c.mgf_tailfac);
         after_launch(c);
         break;
       }
@@ -1686,8 +2098,11 @@ int mgfast_autotune(Ctx &c, int reps, std::string &report) {
   report = "[";
   bool first = true;
   try {
-    // the levels k_f_vtail runs have no line-solve launches to tune
-    for (int l = std::max(2, tail_level(PL) + 1); l <= PL.ngrid; ++l) {
+    // the Thomas levels of k_f_vtail have no line-solve launches to tune; the
+    // levels above them that it takes by tail_level's rule are timed as
+    // launches but stay there (a layout would move them out)
+    const int ltop = tail_level(PL, nprob);
+    for (int l = std::max(2, thomas_levels(PL) + 1); l <= PL.ngrid; ++l) {
       const MgLevel &L = PL.lv[l - 1];
       for (int dir = 0; dir < 2; ++dir) {
         const bool xl = dir == 1;
@@ -1732,8 +2147,10 @@ int mgfast_autotune(Ctx &c, int reps, std::string &report) {
               best_ms = ms;
             }
           }
-        (xl ? PL.lanes_x : PL.lanes_y)[l] = best;
-        (xl ? PL.seg_x : PL.seg_y)[l] = best_seg;
+        if (l > ltop) {
+          (xl ? PL.lanes_x : PL.lanes_y)[l] = best;
+          (xl ? PL.seg_x : PL.seg_y)[l] = best_seg;
+        }
         report += std::string(first ? "" : ", ") + "{\"level\": " + std::to_string(l) + ", \"dir\": \"" +
                   (xl ? "x" : "y") + "\", \"n\": " + std::to_string(n) + ", \"us\": {" + row +
                   "}, \"lanes\": " + std::to_string(best) + ", \"seg\": " + std::to_string(best_seg) + "}";
