@@ -96,64 +96,145 @@ __global__ void k_inject(MgDev g, int level) {  // level -> level-1
 
 // --------------------------------------------------------------------------
 // one point update of relmd2crp
+template <bool ORTH>
 __device__ __forceinline__ double relax_value(const double *ph, size_t si, size_t sj, const double *cof, size_t npt,
-                                              size_t pt, double rhs, double inv9, bool orth) {
+                                              size_t pt, double rhs, double inv9) {
   // ph points at phi(i,j) of this problem; si, sj are the i and j strides
+  // the sum starts from the right-hand side: five or nine FP64 operations a
+  // point, one fewer than forming it apart
   const double c1 = cof[pt], c3 = cof[2 * npt + pt], c5 = cof[4 * npt + pt], c7 = cof[6 * npt + pt];
-  double s;
-  if (orth) {
-    s = c1 * ph[si];
-    s = s + c3 * ph[sj];
-    s = s + c5 * ph[-(long)si];
-    s = s + c7 * ph[-(long)sj];
-  } else {
-    const double c2 = cof[npt + pt], c4 = cof[3 * npt + pt], c6 = cof[5 * npt + pt], c8 = cof[7 * npt + pt];
-    s = c1 * ph[si];
-    s = s + c2 * ph[si + sj];
-    s = s + c3 * ph[sj];
-    s = s + c4 * ph[sj - si];
-    s = s + c5 * ph[-(long)si];
-    s = s + c6 * ph[-(long)(si + sj)];
-    s = s + c7 * ph[-(long)sj];
-    s = s + c8 * ph[si - sj];
-  }
-  return (rhs - s) * inv9;
+  double s = rhs - c1 * ph[si];
+  if (!ORTH) s = s - cof[npt + pt] * ph[si + sj];
+  s = s - c3 * ph[sj];
+  if (!ORTH) s = s - cof[3 * npt + pt] * ph[sj - si];
+  s = s - c5 * ph[-(long)si];
+  if (!ORTH) s = s - cof[5 * npt + pt] * ph[-(long)(si + sj)];
+  s = s - c7 * ph[-(long)sj];
+  if (!ORTH) s = s - cof[7 * npt + pt] * ph[si - sj];
+  return s * inv9;
+}
+
+// The batched kernels below run one grid row a row of the level, its points
+// times the problems over the threads (problem fastest): one 32-bit division
+// finds the point, where flat 64-bit indices took longer than the FP64 work
+// they led to.
+__device__ __forceinline__ bool row_item(unsigned n, int P, int &c, int &p) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned q = t / (unsigned)P;
+  c = (int)q;
+  p = (int)(t - q * (unsigned)P);
+  return q < n;
 }
 
 // first i >= 1 of colour c (1..4) in row j: i + j = c + 1 (mod 4)
-__device__ __forceinline__ int first_i(int c, int j) { return 1 + (((c + 1 - j - 1) % 4) + 4) % 4; }
+__device__ __forceinline__ int first_i(int c, int j) { return 1 + ((c - j) & 3); }
 
 // Fine-level relaxation phase: colour c, row class r (1..4) or all rows
 // (r = 0, orthogonal path).  ghost_on_write: write the periodic ghost
 // columns when i = nx-1 or i = 2 is updated.
+template <bool ORTH>
 __global__ void k_relax_phase(MgDev g, int level, int c, int r, int ghost_on_write) {
   if (*g.alldone) return;
   const LvDev L = g.lv[level - 1];
   const int P = g.P;
   const int nx = L.nx, ny = L.ny;
-  const int ncol = (nx + 3) / 4 + 1;  // columns per row (upper bound)
-  const int nrow = (r == 0) ? ny : (ny - r) / 4 + 1;
-  const long npoint = (long)nrow * ncol;
+  const int j = (r == 0) ? 1 + (int)blockIdx.y : r + 4 * (int)blockIdx.y;
+  const int i0 = first_i(c, j);
+  int coli, p;
+  if (!row_item((nx >= i0) ? (nx - i0) / 4 + 1 : 0, P, coli, p) || g.done[p]) return;
   const size_t npt = (size_t)nx * ny;
   const size_t si = P, sj = (size_t)(nx + 2) * P;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < npoint * P; t += (long)gridDim.x * blockDim.x) {
-    const int p = (int)(t % P);
-    if (g.done[p]) continue;
-    const long q = t / P;
-    const int rowi = (int)(q / ncol), coli = (int)(q % ncol);
-    const int j = (r == 0) ? 1 + rowi : r + 4 * rowi;
-    if (j > ny) continue;
-    const int i = first_i(c, j) + 4 * coli;
-    if (i > nx) continue;
-    const size_t pt = PT(L, i, j);
-    double *ph = &PH(L, P, i, j, p);
-    const double v = relax_value(ph, si, sj, L.cof, npt, pt, L.rhs[pt * P + p], L.inv9[pt * P + p], g.orth);
-    *ph = v;
-    if (ghost_on_write) {
-      if (i == nx - 1) PH(L, P, 0, j, p) = v;
-      if (i == 2) PH(L, P, nx + 1, j, p) = v;
-    }
+  const int i = i0 + 4 * coli;
+  const size_t pt = PT(L, i, j);
+  double *ph = &PH(L, P, i, j, p);
+  const double v = relax_value<ORTH>(ph, si, sj, L.cof, npt, pt, L.rhs[pt * P + p], L.inv9[pt * P + p]);
+  *ph = v;
+  if (ghost_on_write) {
+    if (i == nx - 1) PH(L, P, 0, j, p) = v;
+    if (i == 2) PH(L, P, nx + 1, j, p) = v;
   }
+}
+
+// The same sweeps of one level on a non-orthogonal grid, whole: one block per
+// problem with the problem's phi in shared memory, `count` sweeps of four
+// colours, four row classes and the ghost refresh each, separated by block
+// barriers instead of launches (20 a sweep).  A thread owns at most one point
+// of a phase while the level has at most 16 x its threads, and fetches the
+// next phase's coefficients, right-hand side and reciprocal (which no phase
+// changes) before the barrier; wider levels walk their points.
+// What bounds it: FP64, nine operations a point at 1.7 a clock and SM
+// (12,513 points: 32 us a sweep of one problem), on as many SMs as there are
+// problems; the phase launches spread the points over all SMs but each took
+// 5 us for work of half a microsecond.  Measured, 44 problems of 129 x 97
+// sheared, a batch's fine-level sweeps: 9.0 -> 2.8 ms.
+constexpr int kRelaxThreads = 1024;
+inline size_t relax_block_smem(int nx, int ny) { return sizeof(double) * (size_t)(nx + 2) * (ny + 2); }
+
+__global__ void __launch_bounds__(kRelaxThreads) k_relax_block(MgDev g, int level, int count) {
+  extern __shared__ double sm[];
+  const int p = blockIdx.x;
+  if (*g.alldone || g.done[p]) return;
+  const LvDev L = g.lv[level - 1];
+  const int P = g.P, nx = L.nx, ny = L.ny, npt = nx * ny, sj = nx + 2;
+  const int nph = sj * (ny + 2);
+  const double *rhs = L.rhs + p, *inv9 = L.inv9 + p, *cof = L.cof;
+  double *gphi = L.phi + p;
+  for (int t = threadIdx.x; t < nph; t += kRelaxThreads)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(sm + t)),
+                 "l"(gphi + (size_t)t * P)
+                 : "memory");
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  // phase ph = 0..15: colour 1 + ph / 4, row class 1 + ph % 4
+  double c[8], rv = 0.0, iv = 0.0;
+  int q = 0;  // this thread's point in sm, 0: none
+  auto fetch = [&](int ph, unsigned t) {
+    const int r = 1 + (ph & 3), i0 = first_i(1 + (ph >> 2), r);
+    const unsigned ncol = (nx >= i0) ? (nx - i0) / 4 + 1 : 0, nrow = (ny >= r) ? (ny - r) / 4 + 1 : 0;
+    q = 0;
+    if (t >= nrow * ncol) return;
+    const unsigned a = t / ncol;
+    const int j = r + 4 * (int)a, i = i0 + 4 * (int)(t - a * ncol);
+    const int pt = (j - 1) * nx + (i - 1);
+    q = j * sj + i;
+#pragma unroll
+    for (int l = 0; l < 8; ++l) c[l] = cof[(size_t)l * npt + pt];
+    rv = rhs[(size_t)pt * P];
+    iv = inv9[(size_t)pt * P];
+  };
+  auto update = [&]() {
+    double *ph = sm + q;
+    double s = rv - c[0] * ph[1];
+    s = s - c[1] * ph[1 + sj];
+    s = s - c[2] * ph[sj];
+    s = s - c[3] * ph[sj - 1];
+    s = s - c[4] * ph[-1];
+    s = s - c[5] * ph[-1 - sj];
+    s = s - c[6] * ph[-sj];
+    s = s - c[7] * ph[1 - sj];
+    *ph = s * iv;
+  };
+  const unsigned most = (unsigned)((nx + 3) / 4) * (unsigned)((ny + 3) / 4);
+  fetch(0, threadIdx.x);
+  __syncthreads();
+  for (int sw = 0; sw < count; ++sw)
+    for (int ph = 0; ph < 16; ++ph) {
+      if (q) update();
+      for (unsigned t = threadIdx.x + kRelaxThreads; t < most; t += kRelaxThreads) {
+        fetch(ph, t);
+        if (q) update();
+      }
+      if (sw + 1 < count || ph < 15) fetch((ph + 1) & 15, threadIdx.x);
+      __syncthreads();
+      if ((ph & 3) == 3) {
+        // periodic virtual boundaries after each colour
+        for (int j = 1 + threadIdx.x; j <= ny; j += kRelaxThreads) {
+          sm[j * sj] = sm[j * sj + nx - 1];
+          sm[j * sj + nx + 1] = sm[j * sj + 2];
+        }
+        __syncthreads();
+      }
+    }
+  for (int t = threadIdx.x; t < nph; t += kRelaxThreads) gphi[(size_t)t * P] = sm[t];
 }
 
 // periodic virtual boundaries (mud2cr.f:1784-1789, mudcom.f:540-551)
@@ -161,11 +242,10 @@ __global__ void k_ghost(MgDev g, int level) {
   if (*g.alldone) return;
   const LvDev L = g.lv[level - 1];
   const int P = g.P;
-  const long n = (long)L.ny * P;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int p = (int)(t % P);
-    if (g.done[p]) continue;
-    const int j = 1 + (int)(t / P);
+  int cj, p;
+  if (!row_item(L.ny, P, cj, p) || g.done[p]) return;
+  {
+    const int j = 1 + cj;
     PH(L, P, 0, j, p) = PH(L, P, L.nx - 1, j, p);
     PH(L, P, L.nx + 1, j, p) = PH(L, P, 2, j, p);
   }
@@ -174,34 +254,31 @@ __global__ void k_ghost(MgDev g, int level) {
 // residual on the fine level into the scratch array (resmd2cr,
 // mud2cr.f:1618-1665), then full weighting to the coarse rhs (res2,
 // mudcom.f:120-257) and phic = 0.
+template <bool ORTH>
 __global__ void k_resid(MgDev g, int level) {
   if (*g.alldone) return;
   const LvDev L = g.lv[level - 1];
   const int P = g.P;
   const size_t npt = (size_t)L.nx * L.ny;
   const size_t si = P, sj = (size_t)(L.nx + 2) * P;
-  const long n = (long)npt * P;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int p = (int)(t % P);
-    if (g.done[p]) continue;
-    const long pt = t / P;
-    const int i = 1 + (int)(pt % L.nx), j = 1 + (int)(pt / L.nx);
-    const double *ph = &PH(L, P, i, j, p);
-    const double *cf = L.cof;
-    double s = cf[pt] * ph[si];
-    s = s + cf[npt + pt] * ph[si + sj];
-    s = s + cf[2 * npt + pt] * ph[sj];
-    s = s + cf[3 * npt + pt] * ph[sj - si];
-    s = s + cf[4 * npt + pt] * ph[-(long)si];
-    s = s + cf[5 * npt + pt] * ph[-(long)(si + sj)];
-    s = s + cf[6 * npt + pt] * ph[-(long)sj];
-    s = s + cf[7 * npt + pt] * ph[si - sj];
-    // c9 itself (not its reciprocal) enters the residual
-    const double s4 = cf[8 * npt + pt], corr = cf[9 * npt + pt], jac = cf[10 * npt + pt];
-    const double c9v = ((-g.kx2[p] * jac) - s4) + corr;
-    s = s + c9v * ph[0];
-    g.scr[((size_t)j * (L.nx + 2) + i) * P + p] = L.rhs[pt * P + p] - s;
-  }
+  int ci, p;
+  if (!row_item(L.nx, P, ci, p) || g.done[p]) return;
+  const int i = 1 + ci, j = 1 + (int)blockIdx.y;
+  const size_t pt = PT(L, i, j);
+  const double *ph = &PH(L, P, i, j, p);
+  const double *cf = L.cof + pt;
+  double s = cf[0] * ph[si];
+  if (!ORTH) s = s + cf[npt] * ph[si + sj];
+  s = s + cf[2 * npt] * ph[sj];
+  if (!ORTH) s = s + cf[3 * npt] * ph[sj - si];
+  s = s + cf[4 * npt] * ph[-(long)si];
+  if (!ORTH) s = s + cf[5 * npt] * ph[-(long)(si + sj)];
+  s = s + cf[6 * npt] * ph[-(long)sj];
+  if (!ORTH) s = s + cf[7 * npt] * ph[si - sj];
+  // c9 itself (not its reciprocal) enters the residual
+  const double c9v = ((-g.kx2[p] * cf[10 * npt]) - cf[8 * npt]) + cf[9 * npt];
+  s = s + c9v * ph[0];
+  g.scr[((size_t)j * (L.nx + 2) + i) * P + p] = L.rhs[pt * P + p] - s;
 }
 
 __global__ void k_res2(MgDev g, int level) {  // level -> level-1
@@ -210,14 +287,12 @@ __global__ void k_res2(MgDev g, int level) {  // level -> level-1
   const int P = g.P;
   const int nx = F.nx, ny = F.ny, ncx = C.nx, ncy = C.ny;
   const int ix = (ncx == nx) ? 0 : 1, jy = (ncy == ny) ? 0 : 1;
-  const long n = (long)(ncx + 2) * (ncy + 2) * P;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int p = (int)(t % P);
-    if (g.done[p]) continue;
-    const long q = t / P;
-    const int ic = (int)(q % (ncx + 2)), jc = (int)(q / (ncx + 2));
-    C.phi[q * P + p] = 0.0;
-    if (ic < 1 || ic > ncx || jc < 1 || jc > ncy) continue;
+  int ic, p;
+  if (!row_item(ncx + 2, P, ic, p) || g.done[p]) return;
+  {
+    const int jc = (int)blockIdx.y;
+    PH(C, P, ic, jc, p) = 0.0;
+    if (ic < 1 || ic > ncx || jc < 1 || jc > ncy) return;
     const int i = ic + ix * (ic - 1), j = jc + jy * (jc - 1);
     int im1 = i - 1, ip1 = i + 1, jm1 = j - 1, jp1 = j + 1;
     if (ic == 1 || ic == ncx) {
@@ -264,14 +339,10 @@ __global__ void k_prolong_x(MgDev g, int level, int intpol, int mode) {  // coar
   const int nx = F.nx, ny = F.ny, ncx = C.nx, ncy = C.ny;
   const bool ycoarse = ncy < ny;
   const bool cubic_x = !(intpol == 1 || ncx < 4);
-  const int nrows = ycoarse ? (ny + 1) / 2 : ny;
-  const long n = (long)nrows * (nx + 2) * P;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int pp = (int)(t % P);
-    if (g.done[pp]) continue;
-    const long q = t / P;
-    const int i = (int)(q % (nx + 2));
-    const int rr = (int)(q / (nx + 2));
+  int i, pp;
+  if (!row_item(nx + 2, P, i, pp) || g.done[pp]) return;
+  {
+    const int rr = (int)blockIdx.y;
     const int j = ycoarse ? 2 * rr + 1 : rr + 1;
     const int jc = ycoarse ? j / 2 + 1 : j;
     auto pc = [&](int ic) { return PH(C, P, ic, jc, pp); };
@@ -293,12 +364,10 @@ __global__ void k_prolong_y(MgDev g, int level, int intpol, int mode) {
   const int nx = F.nx, ny = F.ny, ncy = C.ny;
   const bool ycoarse = ncy < ny;
   const bool cubic_y = !(intpol == 1 || ncy < 4);
-  const long n = (long)nx * ny * P;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int pp = (int)(t % P);
-    if (g.done[pp]) continue;
-    const long q = t / P;
-    const int i = 1 + (int)(q % nx), j = 1 + (int)(q / nx);
+  int ci, pp;
+  if (!row_item(nx, P, ci, pp) || g.done[pp]) return;
+  {
+    const int i = 1 + ci, j = 1 + (int)blockIdx.y;
     auto Q = [&](int jj) -> double {
       return (mode == 0) ? g.scr[((size_t)jj * (nx + 2) + i) * P + pp] : PH(F, P, i, jj, pp);
     };
@@ -434,62 +503,84 @@ __global__ void k_check_finish(MgDev g, int iter, int last) {
 // Coarse levels 1..lc: one CTA per problem, everything in shared memory.
 struct CoarseLv {
   int nx, ny;
-  int phi, rhs, inv9, cof;  // offsets (doubles) into shared memory
+  // offsets (doubles) into shared memory; rhs and cof hold rhs / c9 and the
+  // couplings / c9, so that an update is one multiply-add a coupling
+  int phi, rhs, inv9, c9, cof;
 };
 struct CoarseArgs {
   MgDev g;
   const MgOp *ops;
   int nops;
   int intpol;
-  int ncof;  // 4 (orthogonal) or 8
   CoarseLv lv[24];
   int scr;   // scratch offset
   int total; // doubles of shared memory
 };
 
-__device__ void c_relax(const CoarseArgs &A, double *sm, int level, int count, int &stale) {
+constexpr int kCoarseThreads = 256;
+
+// A relaxation phase is a few dozen points whose FP64 chain is what the phase
+// takes: a warp's FP64 instruction holds its quarter of the SM for 64 clocks,
+// however many of its lanes work (measured), so the points are packed over
+// the threads, and while the phase fits four warps that way two lanes share a
+// point's couplings and add their halves.  (One lane a point and the sum and
+// right-hand side scaled last: ten dependent operations, 298 us a launch on
+// 64 x 129 x 97 sheared; now 178.)
+template <bool ORTH>
+__device__ __forceinline__ void c_relax(const CoarseArgs &A, double *sm, int level, int count, int &stale) {
   const CoarseLv &L = A.lv[level - 1];
   const int nx = L.nx, ny = L.ny;
   double *phi = sm + L.phi;
-  const double *rhs = sm + L.rhs, *inv9 = sm + L.inv9, *cf = sm + L.cof;
-  const size_t npt = (size_t)nx * ny;
+  const double *rhs = sm + L.rhs, *cf = sm + L.cof;
+  const int npt = nx * ny;
   const int sj = nx + 2;
-  const bool orth = A.g.orth;
-  const bool onwrite = orth && (nx % 4 != 2);
+  const bool onwrite = ORTH && (nx % 4 != 2);
+  const int wbase = threadIdx.x & ~31;
   for (int sweep = 0; sweep < count; ++sweep) {
     for (int c = 1; c <= 4; ++c) {
-      for (int r = (orth ? 0 : 1); r <= (orth ? 0 : 4); ++r) {
-        const int nrow = (r == 0) ? ny : (ny - r) / 4 + 1;
-        const int ncol = (nx + 3) / 4 + 1;
-        for (int t = threadIdx.x; t < nrow * ncol; t += blockDim.x) {
-          const int rowi = t / ncol, coli = t % ncol;
+      for (int r = (ORTH ? 0 : 1); r <= (ORTH ? 0 : 4); ++r) {
+        // in one row class every row starts at the same column; with all
+        // rows the start moves one column a row, and ncol is the most
+        const unsigned nrow = (r == 0) ? ny : (ny >= r) ? (ny - r) / 4 + 1 : 0;
+        const int i0 = first_i(c, r);
+        const unsigned ncol = (r == 0) ? (nx + 3) / 4 : (nx >= i0) ? (nx - i0) / 4 + 1 : 0;
+        const unsigned items = nrow * ncol;
+        const bool split = 2 * items <= 128u;
+        const int sh = split ? 1 : 0;
+        for (unsigned w = wbase; w < (items << sh); w += blockDim.x) {
+          const unsigned t = (w + (threadIdx.x & 31)) >> sh;
+          const int half = split ? (threadIdx.x & 1) : 0;
+          const unsigned rowi = t / max(ncol, 1u), coli = t - rowi * ncol;
           const int j = (r == 0) ? 1 + rowi : r + 4 * rowi;
-          if (j > ny) continue;
-          const int i = first_i(c, j) + 4 * coli;
-          if (i > nx) continue;
-          const size_t pt = (size_t)(j - 1) * nx + (i - 1);
-          double *ph = phi + j * sj + i;
-          double s;
-          if (orth) {
-            s = cf[pt] * ph[1];
-            s = s + cf[npt + pt] * ph[sj];
-            s = s + cf[2 * npt + pt] * ph[-1];
-            s = s + cf[3 * npt + pt] * ph[-sj];
-          } else {
-            s = cf[pt] * ph[1];
-            s = s + cf[npt + pt] * ph[1 + sj];
-            s = s + cf[2 * npt + pt] * ph[sj];
-            s = s + cf[3 * npt + pt] * ph[sj - 1];
-            s = s + cf[4 * npt + pt] * ph[-1];
-            s = s + cf[5 * npt + pt] * ph[-1 - sj];
-            s = s + cf[6 * npt + pt] * ph[-sj];
-            s = s + cf[7 * npt + pt] * ph[1 - sj];
-          }
-          const double v = (rhs[pt] - s) * inv9[pt];
-          *ph = v;
-          if (onwrite) {
-            if (i == nx - 1) phi[j * sj] = v;
-            if (i == 2) phi[j * sj + nx + 1] = v;
+          const int i = ((r == 0) ? first_i(c, j) : i0) + 4 * coli;
+          const bool on = t < items && i <= nx;
+          const int pt = on ? (j - 1) * nx + (i - 1) : 0;
+          double *ph = phi + (on ? j * sj + i : sj + 1);
+          // lane 0 of a pair takes the couplings ahead (i+1, j+1), lane 1 the
+          // same ones behind: one instruction stream for both
+          constexpr int H = ORTH ? 2 : 4;
+          const double *k = cf + pt + half * (H * npt);
+          const int sg = half ? -1 : 1;
+          auto ahead = [&](double v, const double *kk, int g) {
+            if (ORTH) {
+              v = v - kk[0] * ph[g];
+              return v - kk[npt] * ph[g * sj];
+            }
+            v = v - kk[0] * ph[g];
+            v = v - kk[npt] * ph[g * (1 + sj)];
+            v = v - kk[2 * npt] * ph[g * sj];
+            return v - kk[3 * npt] * ph[g * (sj - 1)];
+          };
+          double v = half ? 0.0 : rhs[pt];
+          v = ahead(v, k, sg);
+          if (split) v += __shfl_xor_sync(0xffffffffu, v, 1);
+          else v = ahead(v, k + H * npt, -1);
+          if (on && !half) {
+            *ph = v;
+            if (onwrite) {
+              if (i == nx - 1) phi[j * sj] = v;
+              if (i == 2) phi[j * sj + nx + 1] = v;
+            }
           }
         }
         __syncthreads();
@@ -506,43 +597,38 @@ __device__ void c_relax(const CoarseArgs &A, double *sm, int level, int count, i
   }
 }
 
-__device__ void c_restrict(const CoarseArgs &A, double *sm, int level, int p) {
+template <bool ORTH>
+__device__ __forceinline__ void c_restrict(const CoarseArgs &A, double *sm, int level) {
   const CoarseLv &F = A.lv[level - 1], &C = A.lv[level - 2];
   const int nx = F.nx, ny = F.ny, ncx = C.nx, ncy = C.ny;
   const double *phi = sm + F.phi, *rhs = sm + F.rhs, *cf = sm + F.cof;
   double *scr = sm + A.scr;
-  const size_t npt = (size_t)nx * ny;
-  const int sj = nx + 2;
-  const LvDev &G = A.g.lv[level - 1];
-  const size_t gnpt = (size_t)G.nx * G.ny;
-  const double kx2 = A.g.kx2[p];
+  const int npt = nx * ny, sj = nx + 2;
+  const double *c9 = sm + F.c9;
   for (int t = threadIdx.x; t < nx * ny; t += blockDim.x) {
     const int i = 1 + t % nx, j = 1 + t / nx;
     const double *ph = phi + j * sj + i;
-    double s;
-    if (A.ncof == 4) {
-      s = cf[t] * ph[1];
-      s = s + cf[npt + t] * ph[sj];
-      s = s + cf[2 * npt + t] * ph[-1];
-      s = s + cf[3 * npt + t] * ph[-sj];
+    double s = rhs[t] - cf[t] * ph[1];
+    if (ORTH) {
+      s = s - cf[npt + t] * ph[sj];
+      s = s - cf[2 * npt + t] * ph[-1];
+      s = s - cf[3 * npt + t] * ph[-sj];
     } else {
-      s = cf[t] * ph[1];
-      s = s + cf[npt + t] * ph[1 + sj];
-      s = s + cf[2 * npt + t] * ph[sj];
-      s = s + cf[3 * npt + t] * ph[sj - 1];
-      s = s + cf[4 * npt + t] * ph[-1];
-      s = s + cf[5 * npt + t] * ph[-1 - sj];
-      s = s + cf[6 * npt + t] * ph[-sj];
-      s = s + cf[7 * npt + t] * ph[1 - sj];
+      s = s - cf[npt + t] * ph[1 + sj];
+      s = s - cf[2 * npt + t] * ph[sj];
+      s = s - cf[3 * npt + t] * ph[sj - 1];
+      s = s - cf[4 * npt + t] * ph[-1];
+      s = s - cf[5 * npt + t] * ph[-1 - sj];
+      s = s - cf[6 * npt + t] * ph[-sj];
+      s = s - cf[7 * npt + t] * ph[1 - sj];
     }
-    const double c9v = ((-kx2 * G.cof[10 * gnpt + t]) - G.cof[8 * gnpt + t]) + G.cof[9 * gnpt + t];
-    s = s + c9v * ph[0];
-    scr[j * sj + i] = rhs[t] - s;
+    scr[j * sj + i] = c9[t] * (s - ph[0]);
   }
   __syncthreads();
   const int ix = (ncx == nx) ? 0 : 1, jy = (ncy == ny) ? 0 : 1;
   double *phic = sm + C.phi;
   double *rhsc = sm + C.rhs;
+  const double *iv = sm + C.inv9;
   for (int t = threadIdx.x; t < (ncx + 2) * (ncy + 2); t += blockDim.x) phic[t] = 0.0;
   for (int t = threadIdx.x; t < ncx * ncy; t += blockDim.x) {
     const int ic = 1 + t % ncx, jc = 1 + t / ncx;
@@ -560,14 +646,14 @@ __device__ void c_restrict(const CoarseArgs &A, double *sm, int level, int p) {
     }
     auto R = [&](int a, int b) { return scr[b * sj + a]; };
     rhsc[t] = (R(im1, jm1) + R(ip1, jm1) + R(im1, jp1) + R(ip1, jp1) +
-               2. * (R(im1, j) + R(ip1, j) + R(i, jm1) + R(i, jp1)) + 4. * R(i, j)) * .0625;
+               2. * (R(im1, j) + R(ip1, j) + R(i, jm1) + R(i, jp1)) + 4. * R(i, j)) * .0625 * iv[t];
   }
   __syncthreads();
 }
 
 // mode 0: cor2 (add); mode 1: FMG prolon2 (overwrite, ghosts of the rows
 // set by prolon1 only)
-__device__ void c_prolong(const CoarseArgs &A, double *sm, int level, int mode, int &stale) {
+__device__ __forceinline__ void c_prolong(const CoarseArgs &A, double *sm, int level, int mode, int &stale) {
   const CoarseLv &F = A.lv[level - 1], &C = A.lv[level - 2];
   const int nx = F.nx, ny = F.ny, ncx = C.nx, ncy = C.ny;
   const bool ycoarse = ncy < ny;
@@ -615,27 +701,31 @@ __device__ void c_prolong(const CoarseArgs &A, double *sm, int level, int mode, 
   __syncthreads();
 }
 
-__global__ void k_coarse(CoarseArgs A) {
+template <bool ORTH>
+__global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
   extern __shared__ double sm[];
   const MgDev &g = A.g;
   const int p = blockIdx.x;
   if (*g.alldone || g.done[p]) return;
   const int P = g.P;
-  // load every coarse level (phi with ghosts, rhs, 1/c9, coefficients)
+  // load every coarse level (phi with ghosts, 1/c9, c9, rhs / c9, couplings / c9)
+  const double kx2 = g.kx2[p];
   for (int l = 1; l <= g.lc; ++l) {
     const CoarseLv &L = A.lv[l - 1];
     const LvDev &G = g.lv[l - 1];
     const int nph = (L.nx + 2) * (L.ny + 2), npt = L.nx * L.ny;
-    for (int t = threadIdx.x; t < nph; t += blockDim.x) sm[L.phi + t] = G.phi[(size_t)t * P + p];
-    for (int t = threadIdx.x; t < npt; t += blockDim.x) {
-      sm[L.rhs + t] = G.rhs[(size_t)t * P + p];
-      sm[L.inv9 + t] = G.inv9[(size_t)t * P + p];
-    }
-    const int ncof = A.ncof;
-    for (int t = threadIdx.x; t < ncof * npt; t += blockDim.x) {
-      const int l8 = t / npt, pt = t % npt;
-      const int src = (ncof == 4) ? 2 * l8 : l8;  // c1,c3,c5,c7 or c1..c8
-      sm[L.cof + t] = G.cof[(size_t)src * npt + pt];
+#pragma unroll 4
+    for (int t = threadIdx.x; t < nph; t += kCoarseThreads) sm[L.phi + t] = G.phi[(size_t)t * P + p];
+#pragma unroll 2
+    for (int t = threadIdx.x; t < npt; t += kCoarseThreads) {
+      const double iv = G.inv9[(size_t)t * P + p];
+      sm[L.rhs + t] = G.rhs[(size_t)t * P + p] * iv;
+      sm[L.inv9 + t] = iv;
+      sm[L.c9 + t] = ((-kx2 * G.cof[(size_t)10 * npt + t]) - G.cof[(size_t)8 * npt + t]) + G.cof[(size_t)9 * npt + t];
+      // c1, c3, c5, c7 or c1..c8
+#pragma unroll
+      for (int q = 0; q < (ORTH ? 4 : 8); ++q)
+        sm[L.cof + q * npt + t] = G.cof[(size_t)(ORTH ? 2 * q : q) * npt + t] * iv;
     }
   }
   __syncthreads();
@@ -643,19 +733,29 @@ __global__ void k_coarse(CoarseArgs A) {
   for (int l = 0; l < 24; ++l) stale[l] = 0;
   for (int o = 0; o < A.nops; ++o) {
     const MgOp op = A.ops[o];
-    if (op.kind == OP_RELAX) c_relax(A, sm, op.level, op.count, stale[op.level - 1]);
-    else if (op.kind == OP_RESTRICT) c_restrict(A, sm, op.level, p);
+    if (op.kind == OP_RELAX) c_relax<ORTH>(A, sm, op.level, op.count, stale[op.level - 1]);
+    else if (op.kind == OP_RESTRICT) c_restrict<ORTH>(A, sm, op.level);
     else if (op.kind == OP_COR2) c_prolong(A, sm, op.level, 0, stale[op.level - 1]);
     else if (op.kind == OP_PROLONG) c_prolong(A, sm, op.level + 1, 1, stale[op.level]);
   }
-  // store phi and rhs of every coarse level
+  // store phi of every coarse level, and the right-hand sides the schedule
+  // may have replaced (level lc's comes from the level above)
   for (int l = 1; l <= g.lc; ++l) {
     const CoarseLv &L = A.lv[l - 1];
     const LvDev &G = g.lv[l - 1];
     const int nph = (L.nx + 2) * (L.ny + 2), npt = L.nx * L.ny;
-    for (int t = threadIdx.x; t < nph; t += blockDim.x) G.phi[(size_t)t * P + p] = sm[L.phi + t];
-    for (int t = threadIdx.x; t < npt; t += blockDim.x) G.rhs[(size_t)t * P + p] = sm[L.rhs + t];
+    for (int t = threadIdx.x; t < nph; t += kCoarseThreads) G.phi[(size_t)t * P + p] = sm[L.phi + t];
+    if (l < g.lc)
+      for (int t = threadIdx.x; t < npt; t += kCoarseThreads) G.rhs[(size_t)t * P + p] = sm[L.rhs + t] * sm[L.c9 + t];
   }
+}
+
+constexpr size_t kRelaxSmem = 220 * 1024;
+// k_relax_block takes the sheared grids' levels whose phi fits a block, while
+// the 20 phase launches of a sweep cost more than the FP64 work that stays on
+// one SM a problem
+bool relax_in_block(const MgPlan &PL, const MgLevel &L, int nprob) {
+  return !PL.orth && relax_block_smem(L.nx, L.ny) <= kRelaxSmem;
 }
 
 unsigned nblk(long n, int bs) {
@@ -855,7 +955,9 @@ void mg_null_mean(Ctx &c, double *phi_finest, int nprob, const double *kx2_dev) 
 void mg_exact_attributes() {
   static std::once_flag once;
   std::call_once(once, [] {
-    EK_CUDA(cudaFuncSetAttribute(k_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    EK_CUDA(cudaFuncSetAttribute(k_coarse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    EK_CUDA(cudaFuncSetAttribute(k_coarse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    EK_CUDA(cudaFuncSetAttribute(k_relax_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRelaxSmem));
   });
 }
 
@@ -879,6 +981,10 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
   g.tol = c.p.mg_tol;
   g.stop_rule = c.p.mg_stop;
   const int bs = 256;
+  // row_item's grid: cols columns of every problem, rows rows
+  auto rowgrid = [&](int cols, int rows) {
+    return dim3((unsigned)(((long)cols * nprob + bs - 1) / bs), (unsigned)rows);
+  };
   cudaStream_t s = c.stream;
   EK_CUDA(cudaMemsetAsync(w.flags, 0, sizeof(int) * (2 * w.pmax + 4), s));
   EK_CUDA(cudaMemsetAsync(w.red, 0, sizeof(double) * (6 * w.pmax + 8), s));
@@ -892,7 +998,7 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
   CoarseArgs A{};
   A.g = g;
   A.intpol = c.p.mg_intpol;
-  A.ncof = PL.orth ? 4 : 8;
+  const int ncof = PL.orth ? 4 : 8;
   int off = 0;
   int maxph = 0;
   for (int l = 1; l <= PL.lc; ++l) {
@@ -902,7 +1008,8 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
     A.lv[l - 1].phi = off; off += (L.nx + 2) * (L.ny + 2);
     A.lv[l - 1].rhs = off; off += L.nx * L.ny;
     A.lv[l - 1].inv9 = off; off += L.nx * L.ny;
-    A.lv[l - 1].cof = off; off += A.ncof * L.nx * L.ny;
+    A.lv[l - 1].c9 = off; off += L.nx * L.ny;
+    A.lv[l - 1].cof = off; off += ncof * L.nx * L.ny;
     maxph = std::max(maxph, (L.nx + 2) * (L.ny + 2));
   }
   A.scr = off;
@@ -945,7 +1052,8 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
         cb += 8.0 * nprob * (2.0 * (Lq.nx + 2) * (Lq.ny + 2) + 3.0 * Lq.nx * Lq.ny);
       }
       KScope ks(c, KC_MG_COARSE, cb);
-      k_coarse<<<nprob, 256, smem, s>>>(A);
+      if (PL.orth) k_coarse<true><<<nprob, kCoarseThreads, smem, s>>>(A);
+      else k_coarse<false><<<nprob, kCoarseThreads, smem, s>>>(A);
       after_launch(c);
       o = e;
       continue;
@@ -976,16 +1084,24 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
       case OP_RELAX: {
         KScope ks(c, KC_MG_RELAX, 32.0 * L.nx * L.ny * nprob * op.count);
         const bool onwrite = PL.orth && (L.nx % 4 != 2);
-        const int ncol = (L.nx + 3) / 4 + 1;
+        if (relax_in_block(PL, L, nprob)) {
+          k_relax_block<<<nprob, kRelaxThreads, relax_block_smem(L.nx, L.ny), s>>>(g, op.level, op.count);
+          after_launch(c);
+          stale[op.level] = 0;
+          break;
+        }
         for (int sw = 0; sw < op.count; ++sw)
           for (int col = 1; col <= 4; ++col) {
             for (int r = (PL.orth ? 0 : 1); r <= (PL.orth ? 0 : 4); ++r) {
-              const int nrow = (r == 0) ? L.ny : (L.ny - r) / 4 + 1;
-              k_relax_phase<<<nblk((long)nrow * ncol * nprob, bs), bs, 0, s>>>(g, op.level, col, r, onwrite ? 1 : 0);
+              const int nrow = (r == 0) ? L.ny : (L.ny >= r) ? (L.ny - r) / 4 + 1 : 0;
+              if (nrow == 0) continue;
+              const dim3 grid = rowgrid((L.nx + 3) / 4, nrow);
+              if (PL.orth) k_relax_phase<true><<<grid, bs, 0, s>>>(g, op.level, col, r, onwrite ? 1 : 0);
+              else k_relax_phase<false><<<grid, bs, 0, s>>>(g, op.level, col, r, onwrite ? 1 : 0);
               after_launch(c);
             }
             if (!onwrite || stale[op.level]) {
-              k_ghost<<<nblk((long)L.ny * nprob, bs), bs, 0, s>>>(g, op.level);
+              k_ghost<<<rowgrid(L.ny, 1), bs, 0, s>>>(g, op.level);
               after_launch(c);
               stale[op.level] = 0;
             }
@@ -995,10 +1111,11 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
       case OP_RESTRICT: {
         const MgLevel &Cq = PL.lv[op.level - 2];
         KScope ks(c, KC_MG_TRANSFER, 8.0 * nprob * (4.0 * L.nx * L.ny + 2.0 * (Cq.nx + 2) * (Cq.ny + 2)));
-        k_resid<<<nblk((long)L.nx * L.ny * nprob, bs), bs, 0, s>>>(g, op.level);
+        if (PL.orth) k_resid<true><<<rowgrid(L.nx, L.ny), bs, 0, s>>>(g, op.level);
+        else k_resid<false><<<rowgrid(L.nx, L.ny), bs, 0, s>>>(g, op.level);
         after_launch(c);
         const MgLevel &C = PL.lv[op.level - 2];
-        k_res2<<<nblk((long)(C.nx + 2) * (C.ny + 2) * nprob, bs), bs, 0, s>>>(g, op.level);
+        k_res2<<<rowgrid(C.nx + 2, C.ny + 2), bs, 0, s>>>(g, op.level);
         after_launch(c);
         break;
       }
@@ -1009,9 +1126,9 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
         const int fine = (op.kind == OP_COR2) ? op.level : op.level + 1;
         const int mode = (op.kind == OP_COR2) ? 0 : 1;
         const MgLevel &F = PL.lv[fine - 1];
-        k_prolong_x<<<nblk((long)(F.ny + 1) * (F.nx + 2) * nprob, bs), bs, 0, s>>>(g, fine, c.p.mg_intpol, mode);
+        k_prolong_x<<<rowgrid(F.nx + 2, PL.lv[fine - 2].ny < F.ny ? (F.ny + 1) / 2 : F.ny), bs, 0, s>>>(g, fine, c.p.mg_intpol, mode);
         after_launch(c);
-        k_prolong_y<<<nblk((long)F.nx * F.ny * nprob, bs), bs, 0, s>>>(g, fine, c.p.mg_intpol, mode);
+        k_prolong_y<<<rowgrid(F.nx, F.ny), bs, 0, s>>>(g, fine, c.p.mg_intpol, mode);
         after_launch(c);
         if (mode == 1 && PL.lv[fine - 2].ny < F.ny) stale[fine] = 1;
         break;
