@@ -225,10 +225,10 @@ __device__ __forceinline__ void dif_fft_any(V *z, int M, const V *tw, bool conj_
 
 // The flux form of the eta/zeta convection plus the GMAT_12 cross diffusion
 // of field a (duct.F90:735-761; the TH version at 1210-1241 has visc =
-// NU/PR) along one x-line, into zr: from the FP32 copies (fin) or FP64.
+// NU/PR) along one x-line, point n to put(n, value): from the FP32 copies (fin) or FP64.
 // b is U2b, followed in memory by U3b (see the launch).
-template <typename T>
-__device__ __forceinline__ void flux_line(T *zr, const FftConst &fc, int k, int j, size_t base, int lane, bool fin,
+template <typename T, typename Put>
+__device__ __forceinline__ void flux_line(Put put, const FftConst &fc, int k, int j, size_t base, int lane, bool fin,
                                           const double *a, const double *b, const float *af, const float *bf,
                                           double visc) {
   const Dims &d = fc.d;
@@ -250,7 +250,7 @@ __device__ __forceinline__ void flux_line(T *zr, const FftConst &fc, int k, int 
       T s2 = h * (T)(double)U3b[c + sK] * (f + fkp) - h * (T)(double)U3b[c] * (f + fkm);
       s1 = -s1 + qv * (g12a * (fpp + fjp - fjm - fpm) - g12b * (fmp + fjp - fjm - fmm));
       s2 = -s2 + qv * (g12c * (fpp + fkp - fmp - fkm) - g12d * (fkp + fpm - fkm - fmm));
-      zr[n] = s1 + s2;
+      put(n, s1 + s2);
     }
   } else {
     const double *F = a, *U2b = b, *U3b = b + d.nphys();
@@ -262,7 +262,7 @@ __device__ __forceinline__ void flux_line(T *zr, const FftConst &fc, int k, int 
       T s2 = h * (T)U3b[c + sK] * (f + fkp) - h * (T)U3b[c] * (f + fkm);
       s1 = -s1 + qv * (g12a * (fpp + fjp - fjm - fpm) - g12b * (fmp + fjp - fjm - fmm));
       s2 = -s2 + qv * (g12c * (fpp + fkp - fmp - fkm) - g12d * (fkp + fpm - fkm - fmm));
-      zr[n] = s1 + s2;
+      put(n, s1 + s2);
     }
   }
 }
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
     else
       for (int n = lane; n < NX; n += 32) zr[n] = jac * (T)args.a[base + n] * (T)args.b[base + n];
   } else {
-    flux_line<T>(zr, fc, k, j, base, lane, fin, args.a, args.b, args.af, args.bf, args.visc);
+    flux_line<T>([&](int n, T v) { zr[n] = v; }, fc, k, j, base, lane, fin, args.a, args.b, args.af, args.bf, args.visc);
   }
   if (args.pro != PRO_LOAD && (args.extra || args.extraf)) {
     // LES additions: jac * tau for a product, the precomputed terms for a flux
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
   if (fuse) {
     T *zr2 = reinterpret_cast<T *>(z2);
     const bool fin2 = kF && args.a2f != nullptr;
-    flux_line<T>(zr2, fc, k, j, base, lane, fin2, args.a2, args.b2, args.a2f, args.b2f, args.visc2);
+    flux_line<T>([&](int n, T v) { zr2[n] = v; }, fc, k, j, base, lane, fin2, args.a2, args.b2, args.a2f, args.b2f, args.visc2);
     if (kF && args.extraf2)
       for (int n = lane; n < NX; n += 32) zr2[n] = zr2[n] + (T)1.0 * (T)args.extraf2[base + n];
     else if (args.extra2)
@@ -495,12 +495,328 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_c2r(FftConst fc, C2rArg
   }
 }
 
-// Launch a transform.  The register form of the FFT pays in the FP32
-// transforms (measured on 512 x 385 x 257: the inverse 0.34 -> 0.23 ms per
+// ---------------------------------------------------------------------------
+// The FP64 transforms.
+//
+// What bounds them: GB300's FP64 pipe, which takes a warp's instruction 64
+// clocks a quarter SM whatever its active lanes (19 clocks an SM, measured).
+// So the work is counted in warp instructions: every lane has a point in
+// every one of them, and there are as few as the passes allow.
+//   - Lines share a warp: a line of M = NX/2 complex points takes M/8 lanes
+//     (M/16 at M = 512), 32 8/M lines a warp, where one line a warp left 16
+//     lanes idle at NX = 64 and 28 at NX = 16.
+//   - The complex transform goes in radix-8 and radix-4 passes in registers,
+//     exchanged through shared memory (M = 256: three passes, 6,144 operations
+//     a line against radix 2's 8,192).
+//   - The split into (and the merge from) the real line's spectrum does modes k
+//     and M - k together, whose sums and twiddle products differ in sign only:
+//     ten or twelve operations for the two against sixteen for each; the scale
+//     1/(2 NX) sits in the split's twiddles as an exponent.
+// Measured: 98,945 lines of NX = 512 forward 2.09 -> 1.60 ms (the operations
+// alone take 1.40), 4,225 lines of NX = 64 inverse 18.5 -> 12.3 us.
+template <int M> struct Fft64 {
+  static constexpr int PTS = (M == 512) ? 16 : 8;  // points a lane
+  static constexpr int G = M / PTS;                // lanes a line
+  static constexpr int LPW = 32 / G;               // lines a warp
+  static constexpr int STRIDE = M + M / 8;         // a line in shared memory, padded
+  // radices of the passes (0: no third pass)
+  static constexpr int R1 = (M == 8 || M == 64 || M >= 128) ? 8 : 4;
+  static constexpr int R2 = (M == 8) ? 0 : (M == 512 || M == 256 || M == 64 || M == 32) ? 8 : 4;
+  static constexpr int R3 = (M == 512) ? 8 : (M == 256 || M == 128) ? 4 : 0;
+};
+// one pad element every 8, so that eight lanes a multiple of 8 elements apart
+// read distinct banks
+__device__ __forceinline__ int pad64(int e) { return e + (e >> 3); }
+
+__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// a times -i (INV: +i)
+template <bool INV>
+__device__ __forceinline__ double2 rot(double2 a) { return INV ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x); }
+
+template <bool INV>
+__device__ __forceinline__ void fft4(double2 &a0, double2 &a1, double2 &a2, double2 &a3) {
+  const double2 t0 = a0 + a2, t1 = a0 - a2, t2 = a1 + a3, t3 = rot<INV>(a1 - a3);
+  a0 = t0 + t2;
+  a1 = t1 + t3;
+  a2 = t0 - t2;
+  a3 = t1 - t3;
+}
+template <bool INV>
+__device__ __forceinline__ void fft8(double2 *a) {
+  constexpr double s = 0.70710678118654752440;
+  double2 e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6], o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
+  fft4<INV>(e0, e1, e2, e3);
+  fft4<INV>(o0, o1, o2, o3);
+  // W^1 and W^3 of order 8 are s (1 -+ i) and s (-1 -+ i): s goes into the sums
+  const double2 p1 = o1 + rot<INV>(o1), r2 = rot<INV>(o2), p3 = rot<INV>(o3) - o3;
+  a[0] = e0 + o0;
+  a[4] = e0 - o0;
+  a[1] = make_double2(fma(s, p1.x, e1.x), fma(s, p1.y, e1.y));
+  a[5] = make_double2(fma(-s, p1.x, e1.x), fma(-s, p1.y, e1.y));
+  a[2] = e2 + r2;
+  a[6] = e2 - r2;
+  a[3] = make_double2(fma(s, p3.x, e3.x), fma(s, p3.y, e3.y));
+  a[7] = make_double2(fma(-s, p3.x, e3.x), fma(-s, p3.y, e3.y));
+}
+
+// One pass of radix R over blocks of B points of every line of the warp,
+// z in place: output k1 of a butterfly takes the place of its input k1, times
+// W_B^(n2 k1).  The last pass (B = R) puts its outputs in natural order, out(q,
+// k1) the index of output k1 of block q.
+template <int M, int R, int B, bool INV, typename Out>
+__device__ __forceinline__ void pass64(double2 *z, const double2 *__restrict__ tw, int g, Out out) {
+  using F = Fft64<M>;
+  constexpr int m = B / R, N = F::PTS / R;  // butterflies a lane
+  double2 a[N][R];
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const int b = g + u * F::G, q = b / m, n2 = b % m;
+#pragma unroll
+    for (int k = 0; k < R; ++k) a[u][k] = z[pad64(q * B + n2 + m * k)];
+    if constexpr (R == 8) fft8<INV>(a[u]);
+    else fft4<INV>(a[u][0], a[u][1], a[u][2], a[u][3]);
+    if constexpr (m > 1) {
+#pragma unroll
+      for (int k = 1; k < R; ++k) {
+        // W_M^t, t = n2 k M / B < M, from the half table
+        const int t = n2 * k * (M / B);
+        double2 w = tw[t & (M / 2 - 1)];
+        if (t >= M / 2) w = make_double2(-w.x, -w.y);
+        if (INV) w.y = -w.y;
+        a[u][k] = cmul(a[u][k], w);
+      }
+    }
+  }
+  if constexpr (m == 1) __syncwarp();  // the outputs of one lane fall on the inputs of others
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const int b = g + u * F::G, q = b / m, n2 = b % m;
+#pragma unroll
+    for (int k = 0; k < R; ++k) z[pad64((m > 1) ? q * B + n2 + m * k : out(q, k))] = a[u][k];
+  }
+  __syncwarp();
+}
+// The warp's lines, each M complex points at z (this lane's line), natural
+// order in and out.
+template <int M, bool INV>
+__device__ __forceinline__ void fft64(double2 *z, const double2 *tw, int g) {
+  using F = Fft64<M>;
+  auto none = [](int, int) { return 0; };
+  __syncwarp();
+  if constexpr (F::R2 == 0 && F::R3 == 0) {
+    pass64<M, F::R1, M, INV>(z, tw, g, [](int, int k) { return k; });
+  } else if constexpr (F::R3 == 0) {
+    pass64<M, F::R1, M, INV>(z, tw, g, none);
+    pass64<M, F::R2, F::R2, INV>(z, tw, g, [](int q, int k) { return q + F::R1 * k; });
+  } else {
+    pass64<M, F::R1, M, INV>(z, tw, g, none);
+    pass64<M, F::R2, M / F::R1, INV>(z, tw, g, none);
+    // block q = k1 R2 + k1'
+    pass64<M, F::R3, F::R3, INV>(z, tw, g, [](int q, int k) {
+      return q / F::R2 + F::R1 * (q % F::R2) + F::R1 * F::R2 * k;
+    });
+  }
+}
+
+// w 2^-e for a twiddle (zero stays zero), on the integer pipe
+__device__ __forceinline__ double scale_tw(double w, int e) {
+  const long long u = __double_as_longlong(w);
+  return (u << 1) ? __longlong_as_double(u - ((long long)e << 52)) : w;
+}
+
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_r2c64(FftConst fc, R2cArgs args) {
+  using F = Fft64<M>;
+  constexpr int NX = 2 * M;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Dims &d = fc.d;
+  const int nk = args.k1 - args.k0 + 1;
+  const int kw = ((int)blockIdx.x * kWarpsPerBlock + warp) * F::LPW;  // the warp's first line
+  if (kw >= nk) return;
+  const int nl = min(F::LPW, nk - kw), k0 = args.k0 + kw;
+  const int j = args.j0 + (int)blockIdx.y;
+  double2 *zw = reinterpret_cast<double2 *>(smem_raw) + (size_t)warp * F::LPW * F::STRIDE;
+  double2 *zw2 = zw + (size_t)kWarpsPerBlock * F::LPW * F::STRIDE;  // the fused flux's lines
+  auto at = [&](double2 *w, int l, int n) -> double & {
+    return reinterpret_cast<double *>(w + l * F::STRIDE + pad64(n >> 1))[n & 1];
+  };
+  if (args.pro == PRO_LOAD) {
+    // flat over the warp's lines (short lines fill the lanes together)
+    for (int t = lane; t < nl * NX; t += 32) at(zw, t / NX, t % NX) = args.a[d.ip(0, k0 + t / NX, j) + t % NX];
+  } else {
+    for (int l = 0; l < nl; ++l) {
+      const int k = k0 + l;
+      const size_t base = d.ip(0, k, j);
+      const double jac = fc.m.jac[d.m2(k, j)];
+      if (args.pro == PRO_PROD)
+        for (int n = lane; n < NX; n += 32) at(zw, l, n) = jac * args.a[base + n] * args.b[base + n];
+      else
+        flux_line<double>([&](int n, double v) { at(zw, l, n) = v; }, fc, k, j, base, lane, false, args.a, args.b,
+                          args.af, args.bf, args.visc);
+      if (args.extra) {
+        // LES additions: jac * tau for a product, the precomputed terms for a flux
+        const double es = (args.pro == PRO_PROD) ? jac : 1.0;
+        for (int n = lane; n < NX; n += 32) at(zw, l, n) += es * args.extra[base + n];
+      }
+      if (args.fuse_flux) {
+        flux_line<double>([&](int n, double v) { at(zw2, l, n) = v; }, fc, k, j, base, lane, false, args.a2, args.b2,
+                          args.a2f, args.b2f, args.visc2);
+        if (args.extra2)
+          for (int n = lane; n < NX; n += 32) at(zw2, l, n) += args.extra2[base + n];
+      }
+    }
+  }
+  const bool fuse = args.fuse_flux != 0;
+  fft64<M, false>(zw + (lane / F::G) * F::STRIDE, fc.tw_m, lane % F::G);
+  if (fuse) fft64<M, false>(zw2 + (lane / F::G) * F::STRIDE, fc.tw_m, lane % F::G);
+  // split: X_k = (s1 + u, d1 + v) / (2 NX), X_{M-k} = (s1 - u, v - d1) / (2 NX)
+  // with s1 = Re(Z_k + Z_{M-k}), d1 = Im(Z_k - Z_{M-k}) and (u, v) the
+  // product of W_NX^k with (Im(Z_k + Z_{M-k}), -Re(Z_k - Z_{M-k}))
+  const int NKX = d.NKX;
+  const double hi = 0.5 * fc.inv_nx;
+  const int he = 1 + 31 - __clz(NX);
+  auto split = [&](const double2 *z, int k, double2 w, double2 &x, double2 &y) {
+    const double2 a = z[pad64(k & (M - 1))], b = z[pad64((M - k) & (M - 1))];
+    const double s1 = a.x + b.x, d1 = a.y - b.y, s2 = a.y + b.y, d2 = a.x - b.x;
+    const double u = w.x * s2 + w.y * d2, v = w.y * s2 - w.x * d2;
+    x = make_double2(fma(hi, s1, u), fma(hi, d1, v));
+    y = make_double2(fma(hi, s1, -u), fma(-hi, d1, v));
+  };
+  auto emit = [&](int l, int kk, double2 x, double2 x2) {
+    cplx_t *dst = args.dst + d.ic(0, k0 + l, j) + kk;
+    if (args.epi == EPI_STORE) {
+      *dst = cplx_t{x.x, x.y};
+      return;
+    }
+    const cplx_t o = *dst;
+    if (args.epi == EPI_ADD) {
+      *dst = cplx_t{o.re + x.x, o.im + x.y};
+    } else {
+      // CF = CF - CIKXP*CS with CIKXP = (0, kx), then the fused flux's X2
+      const double kv = fc.kx[kk];
+      cplx_t r{o.re + kv * x.y, o.im - kv * x.x};
+      if (fuse) r = cplx_t{r.re + x2.x, r.im + x2.y};
+      *dst = r;
+    }
+  };
+  auto pair = [&](int l, int k) {
+    const double2 *z = zw + l * F::STRIDE, *z2 = zw2 + l * F::STRIDE;
+    const bool lo = k <= NKX, up = k > 0 && 2 * k < M && M - k <= NKX;
+    if (!lo && !up) return;
+    double2 w = fc.tw_n[k], x, y, x2 = make_double2(0.0, 0.0), y2 = x2;
+    w = make_double2(scale_tw(w.x, he), scale_tw(w.y, he));
+    split(z, k, w, x, y);
+    if (fuse) split(z2, k, w, x2, y2);
+    if (lo) emit(l, k, x, x2);
+    if (up) emit(l, M - k, y, y2);
+  };
+  // k = 1..M/2 flat over the lines, k = 0 one lane a line
+  for (int t = lane; t < nl * (M / 2); t += 32) pair(t / (M / 2), 1 + t % (M / 2));
+  if (lane < nl) pair(lane, 0);
+  if (args.epi == EPI_STORE || args.zero_hi)
+    for (int l = 0; l < nl; ++l) {
+      cplx_t *dst = args.dst + d.ic(0, k0 + l, j);
+      for (int kk = NKX + 1 + lane; kk <= d.NX2P; kk += 32) dst[kk] = cplx_t{0.0, 0.0};
+    }
+}
+
+template <int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_c2r64(FftConst fc, C2rArgs args) {
+  using F = Fft64<M>;
+  constexpr int NX = 2 * M;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Dims &d = fc.d;
+  const int nk = args.k1 - args.k0 + 1;
+  const int kw = ((int)blockIdx.x * kWarpsPerBlock + warp) * F::LPW;
+  if (kw >= nk) return;
+  const int nl = min(F::LPW, nk - kw), k0 = args.k0 + kw;
+  const int j = args.j0 + (int)blockIdx.y;
+  const int NKX = d.NKX;
+  double2 *zw = reinterpret_cast<double2 *>(smem_raw) + (size_t)warp * F::LPW * F::STRIDE;
+  auto X = [&](int l, int kk) {
+    if (kk > NKX) return make_double2(0.0, 0.0);
+    const size_t c = d.ic(0, k0 + l, j) + kk;
+    cplx_t v = args.src[c];
+    if (args.src2) {
+      const cplx_t w = args.src2[c];
+      v.re = v.re + args.scale2 * w.re;
+      v.im = v.im + args.scale2 * w.im;
+    }
+    if (args.ik) {  // CIKXP * v
+      const double kv = fc.kx[kk], re = v.re;
+      v.re = -(kv * v.im);
+      v.im = kv * re;
+    }
+    if (kk == 0) v.im = 0.0;
+    return make_double2(v.re, v.im);
+  };
+  // merge: Z'_k = (sr - ti, si + tr), Z'_{M-k} = (sr + ti, tr - si) with s, d =
+  // X_k +- conj X_{M-k} and t = d conj(W_NX^k); X_M = 0
+  auto merge = [&](int l, int k) {
+    double2 *z = zw + l * F::STRIDE;
+    const double2 a = X(l, k), w = fc.tw_n[k];
+    double sr = a.x, si = a.y, dr = a.x, di = a.y;
+    if (k > 0 && M - k <= NKX) {
+      const double2 b = X(l, M - k);
+      sr = a.x + b.x;
+      si = a.y - b.y;
+      dr = a.x - b.x;
+      di = a.y + b.y;
+    }
+    const double tr = dr * w.x + di * w.y, ti = di * w.x - dr * w.y;
+    z[pad64(k)] = make_double2(sr - ti, si + tr);
+    if (k > 0 && 2 * k < M) z[pad64(M - k)] = make_double2(sr + ti, tr - si);
+  };
+  for (int t = lane; t < nl * (M / 2); t += 32) merge(t / (M / 2), 1 + t % (M / 2));
+  if (lane < nl) merge(lane, 0);
+  fft64<M, true>(zw + (lane / F::G) * F::STRIDE, fc.tw_m, lane % F::G);
+  for (int t = lane; t < nl * (NX / 2 + 1); t += 32) {
+    // two points at a time; the last pair is the padding
+    const int l = t / (NX / 2 + 1), e = t - l * (NX / 2 + 1);
+    const double2 v = (e < M) ? zw[l * F::STRIDE + pad64(e)] : make_double2(0.0, 0.0);
+    const size_t q = d.ip(0, k0 + l, j) + 2 * e;
+    if (args.dst) {
+      args.dst[q] = v.x;
+      args.dst[q + 1] = v.y;
+    }
+    if (args.dstf) {
+      args.dstf[q] = d2f_bits(v.x);
+      args.dstf[q + 1] = d2f_bits(v.y);
+    }
+  }
+}
+
+// the FP64 launch of nk lines in each of nj rows; false: no such M
+template <int M>
+void run64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs *r, const C2rArgs *c) {
+  using F = Fft64<M>;
+  const dim3 grid((unsigned)((nk + kWarpsPerBlock * F::LPW - 1) / (kWarpsPerBlock * F::LPW)), (unsigned)nj);
+  const size_t smem = sizeof(double2) * F::STRIDE * F::LPW * kWarpsPerBlock * ((r && r->fuse_flux) ? 2 : 1);
+  if (r) k_r2c64<M><<<grid, 32 * kWarpsPerBlock, smem, s>>>(fc, *r);
+  else k_c2r64<M><<<grid, 32 * kWarpsPerBlock, smem, s>>>(fc, *c);
+}
+bool launch64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs *r, const C2rArgs *c) {
+  switch (fc.M) {
+    case 8: run64<8>(nk, nj, s, fc, r, c); return true;
+    case 16: run64<16>(nk, nj, s, fc, r, c); return true;
+    case 32: run64<32>(nk, nj, s, fc, r, c); return true;
+    case 64: run64<64>(nk, nj, s, fc, r, c); return true;
+    case 128: run64<128>(nk, nj, s, fc, r, c); return true;
+    case 256: run64<256>(nk, nj, s, fc, r, c); return true;
+    case 512: run64<512>(nk, nj, s, fc, r, c); return true;
+    default: return false;
+  }
+}
+
+// Launch a transform (FP64 lines of 16 points and more go through launch64).
+// The register form of the FFT pays in the FP32 transforms (measured on 512 x 385 x 257: the inverse 0.34 -> 0.23 ms per
 // launch; the forward ones, since each launch fuses a component's product
-// and flux transforms, 13.9 -> 11.7 ms a step); in the FP64 and float-float
-// ones its extra registers cost more than the shared-memory passes it
-// saves, so they keep the loop.
+// and flux transforms, 13.9 -> 11.7 ms a step); in the float-float ones its
+// extra registers cost more than the shared-memory passes it saves, so they
+// keep the loop.
 template <typename T>
 void run_r2c(dim3 grid, size_t smem, cudaStream_t s, const FftConst &fc, const R2cArgs &a) {
   const unsigned nt = 32 * kWarpsPerBlock;
@@ -536,6 +852,15 @@ void smem_attributes() {
   const int b = 96 * 1024;
   EK_CUDA(cudaFuncSetAttribute(k_r2c<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
   EK_CUDA(cudaFuncSetAttribute(k_c2r<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+  if constexpr (std::is_same_v<T, double>) {
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_r2c64<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+  }
   if constexpr (std::is_same_v<T, float>) {
     EK_CUDA(cudaFuncSetAttribute(k_c2r<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
     EK_CUDA(cudaFuncSetAttribute(k_r2c<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
@@ -601,7 +926,8 @@ void launch_r2c(Ctx &c, const R2cArgs &a) {
   const size_t smem_f = sizeof(float2) * (fc.M + 32) * kWarpsPerBlock * (a.fuse_flux ? 2 : 1);
   if (lp) run_r2c<float>(grid, smem_f, c.stream, fc, a);
   else if (fft_ff(c, a.lowp)) run_r2c<FF>(grid, smem, c.stream, fc, a);
-  else run_r2c<double>(grid, smem, c.stream, fc, a);
+  else if (!launch64(a.k1 - a.k0 + 1, a.j1 - a.j0 + 1, c.stream, fc, &a, nullptr))
+    run_r2c<double>(grid, smem, c.stream, fc, a);
   after_launch(c);
 }
 
@@ -618,7 +944,8 @@ void launch_c2r(Ctx &c, const C2rArgs &a) {
   const size_t smem_f = sizeof(float2) * (fc.M + 32) * kWarpsPerBlock;
   if (fft_lowp(c, a.lowp)) run_c2r<float>(grid, smem_f, c.stream, fc, a);
   else if (fft_ff(c, a.lowp)) run_c2r<FF>(grid, smem, c.stream, fc, a);
-  else run_c2r<double>(grid, smem, c.stream, fc, a);
+  else if (!launch64(a.k1 - a.k0 + 1, a.j1 - a.j0 + 1, c.stream, fc, nullptr, &a))
+    run_c2r<double>(grid, smem, c.stream, fc, a);
   after_launch(c);
 }
 
@@ -729,13 +1056,13 @@ int run_standalone(bool forward, int nx, int nkx, long nlines, const double *in,
     a.pro = PRO_LOAD;
     a.epi = EPI_STORE;
     a.k0 = 0; a.k1 = (int)nlines - 1; a.j0 = 0; a.j1 = 0;
-    run_r2c<double>(grid, smem, s, fc, a);
+    if (!launch64((int)nlines, 1, s, fc, &a, nullptr)) run_r2c<double>(grid, smem, s, fc, a);
   } else {
     C2rArgs a{};
     a.src = reinterpret_cast<const cplx_t *>(in);
     a.dst = out;
     a.k0 = 0; a.k1 = (int)nlines - 1; a.j0 = 0; a.j1 = 0;
-    run_c2r<double>(grid, smem, s, fc, a);
+    if (!launch64((int)nlines, 1, s, fc, nullptr, &a)) run_c2r<double>(grid, smem, s, fc, a);
   }
   EK_CUDA(cudaPeekAtLastError());
   return EK_OK;
