@@ -1607,9 +1607,14 @@ void launch_pline(const FastDev &g, int l, bool xl, int l0, int lstep, int nline
 #undef EK_PLINE
 }
 
-// The layout the solver uses when nothing was tuned: 8-row segments, 32
-// problems per block while a line has at most 32 segments (n <= 287), else 16.
-int default_lanes(int n) { return (pline_segments(n, 8) <= 32) ? 32 : 16; }
+// The layout the solver uses when nothing was tuned: 8-row segments, 16
+// problems per block (to 567 rows; 8 beyond).  Over grids of 128 x 129 x 97 to
+// 512 x 385 x 257, straight and sheared, 16 problems are as fast as 32 or
+// faster at all but one level (129 rows, 21.4 against 20.6 us a sweep; the
+// finest x-lines of the largest 213 against 238, of 64 x 225 x 161 21 against
+// 27), and 8 gain 2 to 5% on the finest x-lines alone and lose 10 to 25% on
+// the short ones.
+int default_lanes(int n) { return (pline_segments(n, 8) <= 64) ? 16 : 8; }
 
 FastDev make_fastdev(Ctx &c, int nprob, const double *kx2_dev) {
   const MgPlan &PL = c.mg;
