@@ -81,34 +81,27 @@ bool supported_bc(const ek_params &p, std::string &why) {
 }
 
 // Thomas factors of every field, substep and direction for the current
-// DELTA_T (they depend on it through TEMP1 = NU*H_BAR(RK_STEP)/2).
+// DELTA_T (k_adi_factors)
 void build_adi_factors(Ctx &c) {
+  const Dims &d = c.d;
   for (int f = 0; f < 4; ++f)
     for (int rk = 1; rk <= 3; ++rk)
       for (int dir = 0; dir < 2; ++dir) {
-        std::vector<double> a, ib, u;
-        adi_factor_host(c, f, rk, dir, c.h_jac, c.h_g11, c.h_g22, a, ib, u);
         AdiFactors &F = c.adi[f][rk][dir];
-        if (!F.a) {
-          F.a = dalloc<double>(c, a.size());
-          F.ib = dalloc<double>(c, ib.size());
-          F.u = dalloc<double>(c, u.size());
-          if (c.p.ff_arith) {
-            F.a2 = dalloc<float2>(c, a.size());
-            F.ib2 = dalloc<float2>(c, ib.size());
-            F.u2 = dalloc<float2>(c, u.size());
-          }
+        if (F.a) continue;
+        F.nline = (dir == 0) ? d.NZ2 : d.NY2;
+        F.nrow = (dir == 0) ? d.NY2 : d.NZ2;
+        const size_t n = (size_t)F.nline * F.nrow;
+        F.a = dalloc<double>(c, n);
+        F.ib = dalloc<double>(c, n);
+        F.u = dalloc<double>(c, n);
+        if (c.p.ff_arith) {
+          F.a2 = dalloc<float2>(c, n);
+          F.ib2 = dalloc<float2>(c, n);
+          F.u2 = dalloc<float2>(c, n);
         }
-        EK_CUDA(cudaMemcpyAsync(F.a, a.data(), sizeof(double) * a.size(), cudaMemcpyHostToDevice, c.stream));
-        EK_CUDA(cudaMemcpyAsync(F.ib, ib.data(), sizeof(double) * ib.size(), cudaMemcpyHostToDevice, c.stream));
-        EK_CUDA(cudaMemcpyAsync(F.u, u.data(), sizeof(double) * u.size(), cudaMemcpyHostToDevice, c.stream));
-        if (F.a2) {
-          split_ff(c, F.a, F.a2, a.size());
-          split_ff(c, F.ib, F.ib2, ib.size());
-          split_ff(c, F.u, F.u2, u.size());
-        }
-        EK_CUDA(cudaStreamSynchronize(c.stream));
       }
+  launch_adi_factors(c);
 }
 
 // DELTA_T and the H_BAR of COURANT_CURV_MPI (duct.F90:3655-3668)
@@ -954,6 +947,8 @@ int ekgpu_set_metrics(ek_ctx *h, const ek_metrics *m) {
     up(c.m.c11, m->cjob_11, 2 * n2); up(c.m.c12, m->cjob_12, 2 * n2);
     up(c.m.c21, m->cjob_21, 2 * n2); up(c.m.c22, m->cjob_22, 2 * n2);
     up(c.m.thbar, m->th_bar, n2);
+    // the copies above are complete before kernels of c.stream read them
+    EK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     step_graphs_clear(c);  // the plan they were captured from is rebuilt below
     if (!c.m.pg) c.m.pg = dalloc<double>(c, 13 * n2);
     launch_metric_tables(c);
@@ -967,9 +962,6 @@ int ekgpu_set_metrics(ek_ctx *h, const ek_metrics *m) {
       if (c.bc_weights == nullptr) c.bc_weights = dalloc<double>(c, w.size());
       EK_CUDA(cudaMemcpy(c.bc_weights, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice));
     }
-    c.h_jac = jac;
-    c.h_g11 = g11;
-    c.h_g22 = g22;
     build_adi_factors(c);
     // multigrid plan
     MgPlan &P = c.mg;

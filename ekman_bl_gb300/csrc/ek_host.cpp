@@ -318,61 +318,6 @@ static void bc_lhs(int field, int dir, const ek_params &p, const Dims &d, int ro
   (void)d;
 }
 
-// Thomas factors (THOMAS_REAL, src/boundary.F90:53-84) of the lines of one
-// field and direction for RK substep rk.  Line index: K for y lines, J for
-// z lines; rows 0..N+1.  Interior rows follow duct.F90 (e.g. 1704-1716 for
-// y, 1795-1805 for z); boundary rows come from bc_lhs; other rows stay at
-// the initial (0, 1, 0).
-void adi_factor_host(const Ctx &c, int field, int rk, int dir, const std::vector<double> &jac,
-                     const std::vector<double> &g11, const std::vector<double> &g22, std::vector<double> &a,
-                     std::vector<double> &ib, std::vector<double> &u) {
-  const Dims &d = c.d;
-  const ek_params &p = c.p;
-  double coef = p.nu * c.H_BAR[rk] / 2.0;
-  if (field == 0) coef = coef / p.pr;
-  const int nline = (dir == 0) ? d.NZ2 : d.NY2;
-  const int nrow = (dir == 0) ? d.NY2 : d.NZ2;
-  const int js = (field == 0) ? d.JST : d.JS, je = (field == 0) ? d.JET : d.JE;
-  const int zs = (field == 0) ? d.ZST : d.ZS, ze = (field == 0) ? d.ZET : d.ZE;
-  a.assign((size_t)nline * nrow, 0.0);
-  ib.assign((size_t)nline * nrow, 1.0);
-  u.assign((size_t)nline * nrow, 0.0);
-  std::vector<double> L(nrow), D(nrow), U(nrow);
-  const BcSet &bs = c.bc[field][dir];
-  for (int l = 0; l < nline; ++l) {
-    const bool active = (dir == 0) ? (l >= zs && l <= ze) : (l >= js && l <= je);
-    if (!active) continue;
-    for (int r = 0; r < nrow; ++r) { L[r] = 0.0; D[r] = 1.0; U[r] = 0.0; }
-    if (dir == 0) {
-      const int k = l;
-      for (int j = js; j <= je; ++j) {
-        L[j] = -coef * g22[d.m3(k, j, 1)];
-        D[j] = jac[d.m2(k, j)] + coef * (g22[d.m3(k, j + 1, 1)] + g22[d.m3(k, j, 1)]);
-        U[j] = -coef * g22[d.m3(k, j + 1, 1)];
-      }
-    } else {
-      const int j = l;
-      for (int k = zs; k <= ze; ++k) {
-        L[k] = -coef * g11[d.m3(k, j, 2)];
-        D[k] = jac[d.m2(k, j)] + coef * (g11[d.m3(k + 1, j, 2)] + g11[d.m3(k, j, 2)]);
-        U[k] = -coef * g11[d.m3(k + 1, j, 2)];
-      }
-    }
-    for (int t = 0; t < bs.n; ++t) bc_lhs(field, dir, p, d, bs.r[t].row, L[bs.r[t].row], D[bs.r[t].row], U[bs.r[t].row]);
-    // forward elimination on the matrix only
-    double B = D[0];
-    ib[(size_t)l * nrow + 0] = 1.0 / B;
-    u[(size_t)l * nrow + 0] = U[0];
-    for (int r = 0; r + 1 < nrow; ++r) {
-      const double aa = -L[r + 1] / B;
-      B = D[r + 1] + aa * U[r];
-      a[(size_t)l * nrow + r + 1] = aa;
-      ib[(size_t)l * nrow + r + 1] = 1.0 / B;
-      u[(size_t)l * nrow + r + 1] = U[r + 1];
-    }
-  }
-}
-
 // n = p*2^(e-1)+1 with p >= 2; prefer the smallest p >= 3.
 bool mg_pick_shape(int n, int &p, int &e) {
   const int m = n - 1;

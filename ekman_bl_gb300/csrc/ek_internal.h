@@ -335,10 +335,8 @@ struct Ctx {
   // sponge_th: SPONGE_SIGMA(0:NY+1), SPONGE_SIGMA_OUT(0:NZ+1), and the
   // mode-0 mean of CU3X over the upper layer with the dynamic-branch flag
   double *sponge_sig = nullptr, *sponge_sig_out = nullptr, *sponge_red = nullptr;
-  // COURANT_CURV_MPI: device minimum of the CFL time steps; host copies of
-  // the metrics the dt-dependent ADI factors are built from
+  // COURANT_CURV_MPI: device minimum of the CFL time steps
   double *cfl_dt = nullptr;
-  std::vector<double> h_jac, h_g11, h_g22;
   GuessState guess;
   // SAVE_STATS_CURVI planes and sums (ek_stats.cu)
   double *stats_buf = nullptr;
@@ -431,9 +429,7 @@ int metrics_from_grid_host(const ek_params *p, const double *xpoint, const doubl
                            double *cjob_21, double *cjob_22, double *th_bar);
 int build_bc_sets(Ctx &c, std::vector<double> &weights, const std::vector<double> &jac,
                   const std::vector<double> &c22);
-void adi_factor_host(const Ctx &c, int field, int rk, int dir, const std::vector<double> &jac,
-                     const std::vector<double> &g11, const std::vector<double> &g22, std::vector<double> &a,
-                     std::vector<double> &ib, std::vector<double> &u);
+void launch_adi_factors(Ctx &c);
 bool mg_pick_shape(int n, int &p, int &e);
 void launch_courant(Ctx &c);
 int les_metrics_from_grid_host(const ek_params *p, const double *xpoint, const double *ypoint, double *g11y,
@@ -528,7 +524,6 @@ inline float *ff_lo(double *field) { return reinterpret_cast<float *>(field); }
 bool inc_fields(const Ctx &c);
 // the total ADI increment of a field: the second float half of its R buffer
 inline float *inc_plane(Ctx &c, double *R) { return reinterpret_cast<float *>(R) + c.d.nphys(); }
-void split_ff(Ctx &c, const double *in, float2 *out, size_t n);
 void les_alloc(Ctx &c);
 void launch_les(Ctx &c, int rk);
 void launch_th_corners(Ctx &c);

@@ -371,14 +371,6 @@ __global__ void k_adi_tab(Dims d, Metrics m, double coef, int sform, double *tab
   }
 }
 
-// A double array split into float-float pairs (hi, lo).
-__global__ void k_split_ff(size_t n, const double *in, float2 *out) {
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    const FF f(in[q]);
-    out[q] = make_float2(f.hi, f.lo);
-  }
-}
-
 // Per-cell weights of one LES ADI sweep (seven planes, ltab[t * n2 + m2(k, j)]):
 //   t0 = -c Gb(lo), t1 = -c Gb(up), t2 = J + c (Gb(up) + Gb(lo))   the plain row
 //   t3 = h Gm(lo),  t4 = h Gm(up)     eddy-viscosity face weights of the row
@@ -1770,6 +1762,125 @@ void launch_face_velocity(Ctx &c) {
   after_launch(c);
 }
 
+// Thomas factors (THOMAS_REAL, src/boundary.F90:53-84) of every field, substep
+// and direction for the current DELTA_T (they depend on it through TEMP1 =
+// NU*H_BAR(RK_STEP)/2): the interior rows of duct.F90:1704-1716 (y lines) and
+// 1795-1805 (z), the boundary rows of APPLY_BC_*, identity rows elsewhere, and
+// the elimination of the matrix.  One thread a line, every line of the 24
+// sweeps in one launch.
+// What bounds it: a row's FP64 division, about a thousand clocks, in series
+// down the line.  COURANT_CURV_MPI changes DELTA_T between steps, and
+// with the factors built on the host and copied a step of 128 x 129 x 97 took
+// 11.5 ms; it takes 8.3.  The operations are rounded one by one, with the
+// multiply-adds the host's compiler formed.
+struct AdiFactorArgs {
+  Dims d;
+  const double *jac, *g11, *g22;
+  double coef[4][4];  // [field][substep]
+  BcSet bc[4][2];
+  AdiFactors f[4][3][2];
+};
+constexpr int kFactChunk = 8;
+
+__global__ void __launch_bounds__(32) k_adi_factors(const __grid_constant__ AdiFactorArgs a) {
+  const Dims &d = a.d;
+  const int dir = blockIdx.y & 1, rk = 1 + (int)(blockIdx.y >> 1) % 3, f = (int)blockIdx.y / 6;
+  const AdiFactors &F = a.f[f][rk - 1][dir];
+  const int l = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (l >= F.nline) return;
+  const int nrow = F.nrow;
+  const int js = (f == 0) ? d.JST : d.JS, je = (f == 0) ? d.JET : d.JE;
+  const int zs = (f == 0) ? d.ZST : d.ZS, ze = (f == 0) ? d.ZET : d.ZE;
+  const bool active = (dir == 0) ? (l >= zs && l <= ze) : (l >= js && l <= je);
+  const int r0 = (dir == 0) ? js : zs, r1 = (dir == 0) ? je : ze;
+  const double coef = a.coef[f][rk];
+  const double *g = (dir == 0) ? a.g22 : a.g11;
+  const BcSet &bs = a.bc[f][dir];
+  auto put = [&](int r, double va, double vi, double vu) {
+    const size_t q = (size_t)l * nrow + r;
+    F.a[q] = va;
+    F.ib[q] = vi;
+    F.u[q] = vu;
+    if (F.a2) {
+      const FF fa(va), fi(vi), fu(vu);
+      F.a2[q] = make_float2(fa.hi, fa.lo);
+      F.ib2[q] = make_float2(fi.hi, fi.lo);
+      F.u2[q] = make_float2(fu.hi, fu.lo);
+    }
+  };
+  if (!active) {
+    for (int r = 0; r < nrow; ++r) put(r, 0.0, 1.0, 0.0);
+    return;
+  }
+  auto face = [&](int r) { return g[(dir == 0) ? d.m3(l, r, 1) : d.m3(r, l, 2)]; };
+  double B = 1.0, Up = 0.0;
+  for (int rc = 0; rc < nrow; rc += kFactChunk) {
+    // the chunk's metrics before the divisions run through it (the face above
+    // the last row is within the metric arrays' extra row)
+    double gf[kFactChunk + 1], jc[kFactChunk];
+#pragma unroll
+    for (int u = 0; u <= kFactChunk; ++u) gf[u] = face(min(rc + u, nrow));
+#pragma unroll
+    for (int u = 0; u < kFactChunk; ++u) {
+      const int r = min(rc + u, nrow - 1);
+      jc[u] = a.jac[(dir == 0) ? d.m2(l, r) : d.m2(r, l)];
+    }
+#pragma unroll 1
+    for (int u = 0; u < kFactChunk; ++u) {
+      const int r = rc + u;
+      if (r >= nrow) break;
+      double L = 0.0, D = 1.0, U = 0.0;
+      double glo = 0.0, gup = 0.0, jr = 0.0;
+#pragma unroll
+      for (int v = 0; v < kFactChunk; ++v)
+        if (v == u) {
+          glo = gf[v];
+          gup = gf[v + 1];
+          jr = jc[v];
+        }
+      if (r >= r0 && r <= r1) {
+        L = -__dmul_rn(coef, glo);
+        U = -__dmul_rn(coef, gup);
+        D = __fma_rn(coef, __dadd_rn(gup, glo), jr);
+      }
+      for (int t = 0; t < bs.n; ++t)
+        if (bs.r[t].row == r) {
+          L = bs.r[t].l;
+          D = bs.r[t].dg;
+          U = bs.r[t].u;
+        }
+      double aa = 0.0;
+      if (r > 0) {
+        aa = __ddiv_rn(-L, B);
+        D = __fma_rn(aa, Up, D);
+      }
+      B = D;
+      Up = U;
+      put(r, aa, __ddiv_rn(1.0, B), U);
+    }
+  }
+}
+
+void launch_adi_factors(Ctx &c) {
+  const Dims &d = c.d;
+  AdiFactorArgs a;
+  a.d = d;
+  a.jac = c.m.jac;
+  a.g11 = c.m.g11;
+  a.g22 = c.m.g22;
+  for (int f = 0; f < 4; ++f) {
+    for (int rk = 1; rk <= 3; ++rk) {
+      double coef = c.p.nu * c.H_BAR[rk] / 2.0;
+      if (f == 0) coef = coef / c.p.pr;
+      a.coef[f][rk] = coef;
+      for (int dir = 0; dir < 2; ++dir) a.f[f][rk - 1][dir] = c.adi[f][rk][dir];
+    }
+    for (int dir = 0; dir < 2; ++dir) a.bc[f][dir] = c.bc[f][dir];
+  }
+  k_adi_factors<<<dim3((unsigned)((std::max(d.NY2, d.NZ2) + 31) / 32), 24), 32, 0, c.stream>>>(a);
+  after_launch(c);
+}
+
 // The tile form takes lines up to kAdiTileRows rows (their rows and factors
 // fill a block's shared memory); longer ones go through k_adi_inc.
 constexpr int kAdiTileRows = 1600;
@@ -2182,13 +2293,6 @@ void rk_init_attributes() {
 namespace ek {
 bool ff_fields(const Ctx &c) { return c.p.ff_arith == 1 && c.p.fft_fp32 == 1 && !les_active(c); }
 bool inc_fields(const Ctx &c) { return c.p.ff_arith == 2 && c.p.fft_fp32 == 1 && !les_active(c); }
-
-void split_ff(Ctx &c, const double *in, float2 *out, size_t n) {
-  if (n == 0) return;
-  const unsigned nb = (unsigned)std::min<size_t>((n + 255) / 256, 4 * 152);
-  k_split_ff<<<nb, 256, 0, c.stream>>>(n, in, out);
-  after_launch(c);
-}
 }  // namespace ek
 
 namespace ek {
