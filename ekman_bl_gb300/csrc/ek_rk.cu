@@ -27,6 +27,30 @@ struct DivBy {
   }
 };
 
+// The spectral kernels' item: mode i of 0..nm-1 and line k of 0..nk-1, flat over
+// the threads of blockIdx.x, row j = blockIdx.y.  GB300's FP64 pipe, which
+// bounds these kernels, takes a warp's instruction 64 clocks whatever its
+// active lanes, so a line's last warp must not run half empty: with 64-thread
+// blocks per line 171 modes filled 89% of the lanes, 43 modes 67%, 22 modes
+// 34%.  Measured, these kernels together a step: 512 x 385 x 257 18.8 -> 17.1 ms,
+// 64 x 65 x 65 292 -> 257 us.
+__device__ __forceinline__ bool mode_item(int nm, int nk, int &i, int &k) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned q = t / (unsigned)nm;
+  k = (int)q;
+  i = (int)(t - q * (unsigned)nm);
+  return q < (unsigned)nk;
+}
+inline dim3 mode_grid(int nm, int nk, int nj) { return dim3((unsigned)(((long)nm * nk + 63) / 64), (unsigned)nj); }
+// x 2^-e of a metric, exact: on the integer pipe for a normal result
+__device__ __forceinline__ double scale_down(double x, int e) {
+  const long long u = __double_as_longlong(x);
+  if ((u << 1) == 0) return x;
+  const int ex = (int)(u >> 52) & 0x7ff;
+  if (ex > e && ex < 0x7ff) return __longlong_as_double(u - ((long long)e << 52));
+  return x * __longlong_as_double((long long)(1023 - e) << 52);
+}
+
 struct SpecArgs {
   Dims d;
   Metrics m;
@@ -125,9 +149,9 @@ __global__ void k_metric_tables(Dims d, Metrics m) {
 
 __global__ void k_spectral_rhs(SpecArgs a) {
   const Dims &d = a.d;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y, j = blockIdx.z;
-  if (i > d.NX2P) return;
+  int i, k;
+  if (!mode_item(d.NX2P + 1, d.NZ2, i, k)) return;
+  const int j = blockIdx.y;
   const size_t q = d.ic(i, k, j);
   const double jac = a.m.jac[d.m2(k, j)];
   const bool vel = (j >= d.JS && j <= d.JE && k >= d.ZS && k <= d.ZE);
@@ -1453,17 +1477,17 @@ __global__ void k_th_corners(Dims d, T *TH, int zmax1, int zmin6) {
 // REM_DIV_CURV face velocities CU2b, CU3b (duct.F90:2511-2522), zero
 // elsewhere (2501-2503); CU3b follows CU2b in memory.
 __global__ void k_rem_faces(Dims d, Metrics m, const cplx_t *CU2, const cplx_t *CU3, cplx_t *CU2b) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y, j = blockIdx.z;
-  if (i > d.NX2P) return;
+  int i, k;
+  if (!mode_item(d.NX2P + 1, d.NZ2, i, k)) return;
+  const int j = blockIdx.y;
   cplx_t *CU3b = CU2b + d.nspec();
   const size_t q = d.ic(i, k, j);
   if (j >= d.JS && j <= d.JE + 1 && k >= d.ZS && k <= d.ZE + 1) {
     const size_t sK = d.LDC, sJ = (size_t)d.LDC * d.NZ2;
-    CU2b[q] = cadd(cscl(0.5 * m.c22[d.m3(k, j, 1)], cadd(CU2[q], CU2[q - sJ])),
-                   cscl(0.5 * m.c21[d.m3(k, j, 1)], cadd(CU3[q], CU3[q - sJ])));
-    CU3b[q] = cadd(cscl(0.5 * m.c11[d.m3(k, j, 2)], cadd(CU3[q], CU3[q - sK])),
-                   cscl(0.5 * m.c12[d.m3(k, j, 2)], cadd(CU2[q], CU2[q - sK])));
+    CU2b[q] = cadd(cscl(scale_down(m.c22[d.m3(k, j, 1)], 1), cadd(CU2[q], CU2[q - sJ])),
+                   cscl(scale_down(m.c21[d.m3(k, j, 1)], 1), cadd(CU3[q], CU3[q - sJ])));
+    CU3b[q] = cadd(cscl(scale_down(m.c11[d.m3(k, j, 2)], 1), cadd(CU3[q], CU3[q - sK])),
+                   cscl(scale_down(m.c12[d.m3(k, j, 2)], 1), cadd(CU2[q], CU2[q - sK])));
   } else {
     CU2b[q] = cplx_t{0.0, 0.0};
     CU3b[q] = cplx_t{0.0, 0.0};
@@ -1476,9 +1500,9 @@ __global__ void k_rem_faces(Dims d, Metrics m, const cplx_t *CU2, const cplx_t *
 // (2631-2651) and phi_bc negates -Re/-Im back.
 __global__ void k_div_rhs(Dims d, const double *kx, const cplx_t *CU1, const cplx_t *CU2b, const double *jacm,
                           double *rhs, int P) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y, j = blockIdx.z;  // full 0..NZ+1, 0..NY+1
-  if (p >= P) return;
+  int p, k;  // full 0..NZ+1, 0..NY+1
+  if (!mode_item(P, d.NZ2, p, k)) return;
+  const int j = blockIdx.y;
   const int I = p >> 1;
   double v = 0.0;
   if (j >= d.JS && j <= d.JE && k >= d.ZS && k <= d.ZE) {
@@ -1502,9 +1526,9 @@ __global__ void k_div_rhs(Dims d, const double *kx, const cplx_t *CU1, const cpl
 __global__ void k_phi_to_cr1(Dims d, const double *phif, int P, cplx_t *CR1, cplx_t *CP, double temp4, double rtemp4,
                              int update_p,
                              int fp32) {
-  const int I = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y, j = blockIdx.z;
-  if (I > d.NX2P) return;
+  int I, k;
+  if (!mode_item(d.NX2P + 1, d.NZ2, I, k)) return;
+  const int j = blockIdx.y;
   cplx_t v{0.0, 0.0};
   if (2 * I + 1 < P) {
     const size_t b = ((size_t)j * d.NZ2 + k) * P + 2 * I;
@@ -1526,9 +1550,10 @@ __global__ void k_phi_to_cr1(Dims d, const double *phif, int P, cplx_t *CR1, cpl
 
 // Face-velocity correction (duct.F90:2709-2724).
 __global__ void k_correct_faces(Dims d, Metrics m, const cplx_t *CR1, cplx_t *CU2b) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = d.ZS + blockIdx.y, j = d.JS + blockIdx.z;
-  if (i > d.NX2P) return;
+  int i, k;
+  if (!mode_item(d.NX2P + 1, d.ZE - d.ZS + 1, i, k)) return;
+  k += d.ZS;
+  const int j = d.JS + blockIdx.y;
   cplx_t *CU3b = CU2b + d.nspec();
   const size_t q = d.ic(i, k, j);
   const size_t sK = d.LDC, sJ = (size_t)d.LDC * d.NZ2;
@@ -1536,8 +1561,8 @@ __global__ void k_correct_faces(Dims d, Metrics m, const cplx_t *CR1, cplx_t *CU
   // the same terms with each metric product fused into its subtraction
   const cplx_t p00 = P(0, 0), p0m = P(0, -1), pm0 = P(-1, 0), pmm = P(-1, -1);
   const cplx_t p10 = P(1, 0), p1m = P(1, -1), p01 = P(0, 1), pm1 = P(-1, 1);
-  const double a22 = m.g22[d.m3(k, j, 1)], a12 = 0.25 * m.g12[d.m3(k, j, 1)];
-  const double b11 = m.g11[d.m3(k, j, 2)], b12 = 0.25 * m.g12[d.m3(k, j, 2)];
+  const double a22 = m.g22[d.m3(k, j, 1)], a12 = scale_down(m.g12[d.m3(k, j, 1)], 2);
+  const double b11 = m.g11[d.m3(k, j, 2)], b12 = scale_down(m.g12[d.m3(k, j, 2)], 2);
   const cplx_t u = CU2b[q], w = CU3b[q];
   CU2b[q] = cplx_t{fma(-a12, ((p10.re + p1m.re) - pm0.re) - pmm.re, fma(-a22, p00.re - p0m.re, u.re)),
                    fma(-a12, ((p10.im + p1m.im) - pm0.im) - pmm.im, fma(-a22, p00.im - p0m.im, u.im))};
@@ -1548,9 +1573,10 @@ __global__ void k_correct_faces(Dims d, Metrics m, const cplx_t *CR1, cplx_t *CU
 // Cell-centre correction (duct.F90:2729-2750).
 __global__ void k_correct_cells(Dims d, Metrics m, const double *kx, const cplx_t *CR1, cplx_t *CU1, cplx_t *CU2,
                                 cplx_t *CU3) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = d.ZS + blockIdx.y, j = d.JS + blockIdx.z;
-  if (i > d.NX2P) return;
+  int i, k;
+  if (!mode_item(d.NX2P + 1, d.ZE - d.ZS + 1, i, k)) return;
+  k += d.ZS;
+  const int j = d.JS + blockIdx.y;
   const size_t q = d.ic(i, k, j);
   const size_t sK = d.LDC, sJ = (size_t)d.LDC * d.NZ2;
   auto P = [&](int dk, int dj) { return CR1[q + (long)dk * (long)sK + (long)dj * (long)sJ]; };
@@ -1570,9 +1596,9 @@ __global__ void k_correct_cells(Dims d, Metrics m, const double *kx, const cplx_
 // Divergence after the projection (duct.F90:2754-2761) into CS.
 __global__ void k_div_check(Dims d, const double *kx, const double *jacm, const cplx_t *CU1, const cplx_t *CU2b,
                             cplx_t *CS) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y, j = blockIdx.z;
-  if (i > d.NX2P) return;
+  int i, k;
+  if (!mode_item(d.NX2P + 1, d.NZ2, i, k)) return;
+  const int j = blockIdx.y;
   const size_t q = d.ic(i, k, j);
   cplx_t v{0.0, 0.0};
   if (j >= d.JS && j <= d.JE && k >= d.ZS && k <= d.ZE) {
@@ -1677,7 +1703,7 @@ void launch_spectral_rhs(Ctx &c, int rk) {
   a.strat_per = (p.v_bc[EK_ZMAX] == 6 && p.u_bc[EK_ZMAX] == 6 && p.w_bc[EK_ZMAX] == 6 && p.ri_tau != 0.0) ? 1 : 0;
   a.reset = (a.strat_per && p.save_stats_int > 0 && (2 * p.time_step) % p.save_stats_int == 0) ? 1 : 0;
   a.d = spec_dims(c);
-  dim3 grid((a.d.NX2P + 1 + 63) / 64, c.d.NZ2, c.d.NY2);
+  const dim3 grid = mode_grid(a.d.NX2P + 1, c.d.NZ2, c.d.NY2);
   KScope ks(c, KC_SPECTRAL, 16.0 * c.d.nspec() * (a.d.NX2P + 1.0) / c.d.LDC * (5 + (rk > 1 ? 4 : 0) + 8));
   if (a.sponge) {
     const int nys = (p.ny_s_t > p.ny) ? (2 * p.ny) / 3 : p.ny_s_t;
@@ -2166,10 +2192,10 @@ void launch_divergence_rhs(Ctx &c, double *rhs, int P) {
   const Dims ds = spec_dims(c);
   const double fm = (ds.NX2P + 1.0) / d.LDC;  // share of the modes processed
   KScope ks(c, KC_DIVERGENCE, 16.0 * d.nspec() * fm * 4 + (16.0 * d.nspec() * 3 + 8.0 * P * d.NZ2 * d.NY2));
-  dim3 g1((ds.NX2P + 1 + 63) / 64, d.NZ2, d.NY2);
+  const dim3 g1 = mode_grid(ds.NX2P + 1, d.NZ2, d.NY2);
   k_rem_faces<<<g1, 64, 0, c.stream>>>(ds, c.m, c.CU2, c.CU3, c.CU2b);
   after_launch(c);
-  dim3 g2((P + 63) / 64, d.NZ2, d.NY2);
+  const dim3 g2 = mode_grid(P, d.NZ2, d.NY2);
   k_div_rhs<<<g2, 64, 0, c.stream>>>(d, c.kx, c.CU1, c.CU2b, c.m.jac, rhs, P);
   after_launch(c);
 }
@@ -2179,13 +2205,13 @@ void launch_projection(Ctx &c, const double *phif, int P, double temp4, bool upd
   const bool side = c.graph_slot >= 0 && !c.timing;
   const Dims ds = spec_dims(c);
   const double fm = (ds.NX2P + 1.0) / d.LDC;
-  dim3 g0((ds.NX2P + 1 + 63) / 64, d.NZ2, d.NY2);
+  const dim3 g0 = mode_grid(ds.NX2P + 1, d.NZ2, d.NY2);
   {
   KScope ks(c, KC_PROJECTION, (16.0 * d.nspec() * (1 + 1 + (update_p ? 2 : 0)) + 16.0 * d.nspec() * (5 + 7 + 4)) * fm);
   k_phi_to_cr1<<<g0, 64, 0, c.stream>>>(ds, phif, P, c.CR1, c.CP, temp4, 1.0 / temp4, update_p ? 1 : 0,
                                        c.p.quirk_phi_fp32);
   after_launch(c);
-  dim3 g1((ds.NX2P + 1 + 63) / 64, d.ZE - d.ZS + 1, d.JE - d.JS + 1);
+  const dim3 g1 = mode_grid(ds.NX2P + 1, d.ZE - d.ZS + 1, d.JE - d.JS + 1);
   k_correct_faces<<<g1, 64, 0, c.stream>>>(ds, c.m, c.CR1, c.CU2b);
   after_launch(c);
   k_correct_cells<<<g1, 64, 0, c.stream>>>(ds, c.m, c.kx, c.CR1, c.CU1, c.CU2, c.CU3);
