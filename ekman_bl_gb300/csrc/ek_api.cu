@@ -950,6 +950,11 @@ int ekgpu_set_metrics(ek_ctx *h, const ek_metrics *m) {
     // the copies above are complete before kernels of c.stream read them
     EK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     step_graphs_clear(c);  // the plan they were captured from is rebuilt below
+    // on an orthogonal grid the step's kernels leave out the terms that these
+    // weights multiply: x + 0 y is x for every finite y, so the results stay
+    c.orth = true;
+    for (size_t t = 0; t < 2 * n2 && c.orth; ++t)
+      c.orth = m->gmat_12[t] == 0.0 && m->cjob_12[t] == 0.0 && m->cjob_21[t] == 0.0;
     if (!c.m.pg) c.m.pg = dalloc<double>(c, 13 * n2);
     launch_metric_tables(c);
     c.les.tab_ok = false;

@@ -295,6 +295,7 @@ struct Ctx {
   float2 *tw_mf = nullptr, *tw_nf = nullptr;  // the same, rounded to FP32
   float4 *tw_mff = nullptr, *tw_nff = nullptr;  // and as float-float pairs
   Metrics m{};
+  bool orth = false;  // every GMAT_12, CJOB_12 and CJOB_21 is zero
   // spectral fields (complex)
   cplx_t *CU1, *CU2, *CU3, *CP, *CTH, *CF1, *CF2, *CF3, *CFTH, *CR1, *CR2, *CR3, *CRTH, *CS, *CU2b, *CU3b;
   // physical fields
