@@ -818,6 +818,14 @@ void run64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs *r,
   else k_c2r64<M><<<grid, 32 * kWarpsPerBlock, smem, s>>>(fc, *c);
 }
 bool launch64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs *r, const C2rArgs *c) {
+  // Few lines leave the GPU idle, and what counts is one warp's chain of FP64
+  // instructions: spread over a whole warp a line has fewer.  1,000 lines,
+  // forward: NX = 16 7.9 us against 13.6, NX = 64 8.3 against 12.4, NX = 128
+  // 10.3 against 14.4; 2,000 lines: equal at NX = 64 and 128; NX = 256 12.3
+  // against 14.4 at 500 and 16.4 against 14.4 at 1,000; from NX = 512 on packed
+  // lines are ahead with 260 lines as well (16.4 us against 20.5).
+  const long lines = (long)nk * nj;
+  if (fc.M <= 128 && lines < 2000 && lines * 2 * fc.M < 180000) return false;
   switch (fc.M) {
     case 8: run64<8>(nk, nj, s, fc, r, c); return true;
     case 16: run64<16>(nk, nj, s, fc, r, c); return true;
@@ -830,7 +838,7 @@ bool launch64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs 
   }
 }
 
-// Launch a transform (FP64 lines of 16 points and more go through launch64).
+// Launch a transform with one line a warp (launch64 takes most FP64 ones).
 // The register form of the FFT pays in the FP32 transforms (measured on 512 x 385 x 257: the inverse 0.34 -> 0.23 ms per
 // launch; the forward ones, since each launch fuses a component's product
 // and flux transforms, 13.9 -> 11.7 ms a step); in the float-float ones its

@@ -38,3 +38,10 @@ def test_transforms_match_numpy(nx, lines):
         b = d.cpu().numpy()
         assert np.all(b[:, nx:] == 0)
         assert np.linalg.norm(b[:, :nx] - ref) <= tol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("nx", [16, 64, 128, 256])
+@pytest.mark.parametrize("lines", [701, 709, 1999, 2001])
+def test_line_counts_about_the_packing_rule(nx, lines):
+    """Both forms on either side of the line count that chooses between them."""
+    test_transforms_match_numpy(nx, lines)
