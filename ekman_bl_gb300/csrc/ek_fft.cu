@@ -225,69 +225,104 @@ __device__ __forceinline__ void dif_fft_any(V *z, int M, const V *tw, bool conj_
 }
 
 // The flux form of the eta/zeta convection plus the GMAT_12 cross diffusion
-// of field a (duct.F90:735-761; the TH version at 1210-1241 has visc =
-// NU/PR) along one x-line, point n to put(n, value): from the FP32 copies (fin) or FP64.
-// b is U2b, followed in memory by U3b (see the launch).
-// fc.orth: GMAT_12 is zero, and the cross diffusion with its four corner
-// loads is left out, for the whole line at once, so that either loop's loads
-// stay together.  The step's forward transforms: FP32 on 512 x 385 x 257
-// 9.9 -> 8.7 ms, FP64 on 256 x 257 x 193 23.2 -> 18.1 ms.
-template <typename T, typename Put>
-__device__ __forceinline__ void flux_line(Put put, const FftConst &fc, int k, int j, size_t base, int lane, bool fin,
-                                          const double *a, const double *b, const float *af, const float *bf,
-                                          double visc) {
+// of a field (duct.F90:735-761; the TH version at 1210-1241 has visc =
+// NU/PR) at one point from the field's neighbours and the face velocities.
+// ORTH: GMAT_12 is zero, and the cross diffusion with its four corner values is
+// left out.  The step's forward transforms: FP32 on 512 x 385 x 257 9.9 ->
+// 8.7 ms, FP64 on 256 x 257 x 193 23.2 -> 18.1 ms.
+template <typename T>
+struct FluxG12 {
+  T a, b, c, d, qv;
+  __device__ FluxG12(const FftConst &fc, int k, int j, double visc)
+      : a(from_f64<T>(fc.m.g12[fc.d.m3(k + 1, j, 2)])), b(from_f64<T>(fc.m.g12[fc.d.m3(k, j, 2)])),
+        c(from_f64<T>(fc.m.g12[fc.d.m3(k, j + 1, 1)])), d(from_f64<T>(fc.m.g12[fc.d.m3(k, j, 1)])),
+        qv(from_f64<T>(0.25 * visc)) {}
+};
+template <typename T>
+__device__ __forceinline__ T flux_orth(T f, T fkp, T fkm, T fjp, T fjm, T u2, T u2p, T u3, T u3p) {
+  const T h = (T)0.5;
+  const T s1 = h * u2p * (f + fjp) - h * u2 * (f + fjm);
+  const T s2 = h * u3p * (f + fkp) - h * u3 * (f + fkm);
+  return -s1 - s2;
+}
+template <typename T>
+__device__ __forceinline__ T flux_gen(const FluxG12<T> &g, T f, T fkp, T fkm, T fjp, T fjm, T fpp, T fpm, T fmp, T fmm,
+                                      T u2, T u2p, T u3, T u3p) {
+  const T h = (T)0.5;
+  T s1 = h * u2p * (f + fjp) - h * u2 * (f + fjm);
+  T s2 = h * u3p * (f + fkp) - h * u3 * (f + fkm);
+  s1 = -s1 + g.qv * (g.a * (fpp + fjp - fjm - fpm) - g.b * (fmp + fjp - fjm - fmm));
+  s2 = -s2 + g.qv * (g.c * (fpp + fkp - fmp - fkm) - g.d * (fkp + fpm - fkm - fmm));
+  return s1 + s2;
+}
+// Two consecutive values in the arithmetic type: one 8-byte load of an FP32
+// plane (a plane's lines start on even elements)
+template <typename T> struct Two {
+  T x, y;
+};
+template <typename T> __device__ __forceinline__ Two<T> two(const float *p) {
+  const float2 v = *reinterpret_cast<const float2 *>(p);
+  return Two<T>{(T)(double)v.x, (T)(double)v.y};
+}
+template <typename T> __device__ __forceinline__ Two<T> two(const double *p) { return Two<T>{(T)p[0], (T)p[1]}; }
+// The flux at points c and c + 1, its loads apart from its value so that
+// several pairs' loads can go out together; b is U2b, followed in memory by U3b
+// (see the launch).
+template <typename T> struct FluxIn {
+  Two<T> f, kp, km, jp, jm, u2, u2p, u3, u3p, pp, pm, mp, mm;
+};
+template <typename T, bool ORTH, typename P>
+__device__ __forceinline__ FluxIn<T> flux_load(const Dims &d, size_t c, const P *F, const P *U2b) {
+  const size_t sK = d.LDX, sJ = (size_t)d.LDX * d.NZ2;
+  const P *U3b = U2b + d.nphys();
+  FluxIn<T> v;
+  v.f = two<T>(F + c), v.kp = two<T>(F + c + sK), v.km = two<T>(F + c - sK);
+  v.jp = two<T>(F + c + sJ), v.jm = two<T>(F + c - sJ);
+  v.u2 = two<T>(U2b + c), v.u2p = two<T>(U2b + c + sJ), v.u3 = two<T>(U3b + c), v.u3p = two<T>(U3b + c + sK);
+  if constexpr (!ORTH) {
+    v.pp = two<T>(F + c + sK + sJ), v.pm = two<T>(F + c + sK - sJ);
+    v.mp = two<T>(F + c - sK + sJ), v.mm = two<T>(F + c - sK - sJ);
+  }
+  return v;
+}
+template <bool ORTH, typename T>
+__device__ __forceinline__ Two<T> flux_value(const FluxG12<T> &g, const FluxIn<T> &v) {
+  if constexpr (ORTH)
+    return Two<T>{flux_orth(v.f.x, v.kp.x, v.km.x, v.jp.x, v.jm.x, v.u2.x, v.u2p.x, v.u3.x, v.u3p.x),
+                  flux_orth(v.f.y, v.kp.y, v.km.y, v.jp.y, v.jm.y, v.u2.y, v.u2p.y, v.u3.y, v.u3p.y)};
+  else
+    return Two<T>{flux_gen(g, v.f.x, v.kp.x, v.km.x, v.jp.x, v.jm.x, v.pp.x, v.pm.x, v.mp.x, v.mm.x, v.u2.x, v.u2p.x,
+                           v.u3.x, v.u3p.x),
+                  flux_gen(g, v.f.y, v.kp.y, v.km.y, v.jp.y, v.jm.y, v.pp.y, v.pm.y, v.mp.y, v.mm.y, v.u2.y, v.u2p.y,
+                           v.u3.y, v.u3p.y)};
+}
+// The same along one x-line, point n to put(n, value), for the FP64 kernel.
+// The choice is made for a whole line at once, so that either loop's loads
+// stay together.
+template <typename Put>
+__device__ __forceinline__ void flux_line(Put put, const FftConst &fc, int k, int j, size_t base, int lane,
+                                          const double *F, const double *U2b, double visc) {
   const Dims &d = fc.d;
   const int NX = d.NX;
-  const T g12a = from_f64<T>(fc.m.g12[d.m3(k + 1, j, 2)]), g12b = from_f64<T>(fc.m.g12[d.m3(k, j, 2)]);
-  const T g12c = from_f64<T>(fc.m.g12[d.m3(k, j + 1, 1)]), g12d = from_f64<T>(fc.m.g12[d.m3(k, j, 1)]);
-  const T qv = from_f64<T>(0.25 * visc);
-  const T h = (T)0.5;
   const size_t sK = d.LDX, sJ = (size_t)d.LDX * d.NZ2;
+  const double *U3b = U2b + d.nphys();
   if (fc.orth) {
-    auto line = [&](auto *F, auto *U2b, auto *U3b) {
-      auto ld = [](auto x) { return sizeof(x) == 4 ? (T)(double)x : (T)x; };
-      for (int n = lane; n < NX; n += 32) {
-        const size_t c = base + n;
-        const T f = ld(F[c]), fkp = ld(F[c + sK]), fkm = ld(F[c - sK]), fjp = ld(F[c + sJ]), fjm = ld(F[c - sJ]);
-        const T s1 = h * ld(U2b[c + sJ]) * (f + fjp) - h * ld(U2b[c]) * (f + fjm);
-        const T s2 = h * ld(U3b[c + sK]) * (f + fkp) - h * ld(U3b[c]) * (f + fkm);
-        put(n, -s1 - s2);
-      }
-    };
-    if (fin) line(af, bf, bf + d.nphys());
-    else line(a, b, b + d.nphys());
+    for (int n = lane; n < NX; n += 32) {
+      const size_t c = base + n;
+      put(n, flux_orth(F[c], F[c + sK], F[c - sK], F[c + sJ], F[c - sJ], U2b[c], U2b[c + sJ], U3b[c], U3b[c + sK]));
+    }
     return;
   }
-  if (fin) {
-    const float *F = af, *U2b = bf, *U3b = bf + d.nphys();
-    for (int n = lane; n < NX; n += 32) {
-      const size_t c = base + n;
-      const T f = (T)(double)F[c], fkp = (T)(double)F[c + sK], fkm = (T)(double)F[c - sK];
-      const T fjp = (T)(double)F[c + sJ], fjm = (T)(double)F[c - sJ];
-      const T fpp = (T)(double)F[c + sK + sJ], fpm = (T)(double)F[c + sK - sJ];
-      const T fmp = (T)(double)F[c - sK + sJ], fmm = (T)(double)F[c - sK - sJ];
-      T s1 = h * (T)(double)U2b[c + sJ] * (f + fjp) - h * (T)(double)U2b[c] * (f + fjm);
-      T s2 = h * (T)(double)U3b[c + sK] * (f + fkp) - h * (T)(double)U3b[c] * (f + fkm);
-      s1 = -s1 + qv * (g12a * (fpp + fjp - fjm - fpm) - g12b * (fmp + fjp - fjm - fmm));
-      s2 = -s2 + qv * (g12c * (fpp + fkp - fmp - fkm) - g12d * (fkp + fpm - fkm - fmm));
-      put(n, s1 + s2);
-    }
-  } else {
-    const double *F = a, *U2b = b, *U3b = b + d.nphys();
-    for (int n = lane; n < NX; n += 32) {
-      const size_t c = base + n;
-      const T f = (T)F[c], fkp = (T)F[c + sK], fkm = (T)F[c - sK], fjp = (T)F[c + sJ], fjm = (T)F[c - sJ];
-      const T fpp = (T)F[c + sK + sJ], fpm = (T)F[c + sK - sJ], fmp = (T)F[c - sK + sJ], fmm = (T)F[c - sK - sJ];
-      T s1 = h * (T)U2b[c + sJ] * (f + fjp) - h * (T)U2b[c] * (f + fjm);
-      T s2 = h * (T)U3b[c + sK] * (f + fkp) - h * (T)U3b[c] * (f + fkm);
-      s1 = -s1 + qv * (g12a * (fpp + fjp - fjm - fpm) - g12b * (fmp + fjp - fjm - fmm));
-      s2 = -s2 + qv * (g12c * (fpp + fkp - fmp - fkm) - g12d * (fkp + fpm - fkm - fmm));
-      put(n, s1 + s2);
-    }
+  const FluxG12<double> g(fc, k, j, visc);
+  for (int n = lane; n < NX; n += 32) {
+    const size_t c = base + n;
+    put(n, flux_gen(g, F[c], F[c + sK], F[c - sK], F[c + sJ], F[c - sJ], F[c + sK + sJ], F[c + sK - sJ],
+                    F[c - sK + sJ], F[c - sK - sJ], U2b[c], U2b[c + sJ], U3b[c], U3b[c + sK]));
   }
 }
 
-// The FP32 register form asks for 8 blocks an SM (64 registers; 72 left 7): the step's forward transforms 10.6 -> 9.8 ms
+// The FP32 register form asks for 8 blocks an SM (64 registers, a 16-byte
+// spill; 72 registers left 7): the step's forward transforms 10.6 -> 9.8 ms
 // on 512 x 385 x 257.  A minimum of 0 leaves the other forms' allocation
 // as the compiler chooses it.
 template <typename T, int E>
@@ -305,55 +340,96 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
   if (kw >= nk) return;
   const int k = args.k0 + kw;
   const int j = args.j0 + (int)blockIdx.y;
-  const int NX = d.NX, M = fc.M;
+  const int M = fc.M;
   V *z = smem_c + (size_t)warp * fstride<E>(M);
-  T *zr = reinterpret_cast<T *>(z);
   const size_t base = d.ip(0, k, j);
   constexpr bool kF = sizeof(T) == 4;
   const bool fin = kF && args.af != nullptr;  // FP32 copies of the inputs
+  // Points go two at a time, and the loads of U pairs go out before any of them
+  // is used: a load a turn leaves the memory waiting.
+  auto batch = [&](auto U_, auto load, auto use) {
+    constexpr int U = decltype(U_)::value, B = (E > 0 && E < U) ? E : U;
+    for (int m0 = lane; m0 < M; m0 += 32 * B) {
+      decltype(load(0)) v[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (E > 0 || m0 + 32 * u < M) v[u] = load(m0 + 32 * u);
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (E > 0 || m0 + 32 * u < M) use(m0 + 32 * u, v[u]);
+    }
+  };
+  constexpr std::integral_constant<int, 4> U4{};
+  auto store = [&](int m, Two<T> v) { z[m] = Cx<T>::make(v.x, v.y); };
+  auto flux = [&](V *y, auto *F, auto *b, double visc) {
+    const FluxG12<T> g(fc, k, j, visc);
+    auto line = [&](auto ORTH) {
+      constexpr bool O = decltype(ORTH)::value;
+      // a general pair is 26 values, an orthogonal one 18
+      constexpr std::integral_constant<int, (kF && O) ? 2 : 1> UF{};
+      batch(UF, [&](int m) { return flux_load<T, O>(d, base + 2 * m, F, b); },
+            [&](int m, const FluxIn<T> &v) {
+              const Two<T> f = flux_value<O>(g, v);
+              y[m] = Cx<T>::make(f.x, f.y);
+            });
+    };
+    if (fc.orth) line(std::true_type{});
+    else line(std::false_type{});
+  };
+  auto add = [&](V *y, auto *x, T es) {
+    batch(U4, [&](int m) { return two<T>(x + base + 2 * m); },
+          [&](int m, Two<T> v) {
+            const V o = y[m];
+            y[m] = Cx<T>::make(o.x + es * v.x, o.y + es * v.y);
+          });
+  };
   if (args.pro == PRO_LOAD) {
+    bool pairs = false;
     if constexpr (std::is_same_v<T, FF>) {
-      if (args.alo) {
-        // a float-float field: the pair as it is, no FP64 split
-        for (int n = lane; n < NX; n += 32) zr[n] = FF(args.af[base + n], args.alo[base + n]);
-      } else {
-        for (int n = lane; n < NX; n += 32) zr[n] = (T)args.a[base + n];
-      }
-    } else if (fin) {
-      // an FP32 field (the increment of the state)
-      for (int n = lane; n < NX; n += 32) zr[n] = (T)args.af[base + n];
-    } else {
-      for (int n = lane; n < NX; n += 32) zr[n] = (T)args.a[base + n];
+      // a float-float field: the pair as it is, no FP64 split
+      pairs = args.alo != nullptr;
+      if (pairs)
+        batch(U4, [&](int m) {
+          const float2 h = *reinterpret_cast<const float2 *>(args.af + base + 2 * m);
+          const float2 l = *reinterpret_cast<const float2 *>(args.alo + base + 2 * m);
+          return Two<T>{FF(h.x, l.x), FF(h.y, l.y)};
+        }, store);
+    }
+    // fin: an FP32 field (the increment of the state)
+    if (!pairs) {
+      if (fin) batch(U4, [&](int m) { return two<T>(args.af + base + 2 * m); }, store);
+      else batch(U4, [&](int m) { return two<T>(args.a + base + 2 * m); }, store);
     }
   } else if (args.pro == PRO_PROD) {
     const T jac = from_f64<T>(fc.m.jac[d.m2(k, j)]);
-    if (fin)
-      for (int n = lane; n < NX; n += 32) zr[n] = jac * (T)(double)args.af[base + n] * (T)(double)args.bf[base + n];
-    else
-      for (int n = lane; n < NX; n += 32) zr[n] = jac * (T)args.a[base + n] * (T)args.b[base + n];
+    auto prod = [&](auto *a, auto *b) {
+      struct In {
+        Two<T> a, b;
+      };
+      batch(U4, [&](int m) { return In{two<T>(a + base + 2 * m), two<T>(b + base + 2 * m)}; },
+            [&](int m, const In &v) { z[m] = Cx<T>::make(jac * v.a.x * v.b.x, jac * v.a.y * v.b.y); });
+    };
+    if (fin) prod(args.af, args.bf);
+    else prod(args.a, args.b);
   } else {
-    flux_line<T>([&](int n, T v) { zr[n] = v; }, fc, k, j, base, lane, fin, args.a, args.b, args.af, args.bf, args.visc);
+    if (fin) flux(z, args.af, args.bf, args.visc);
+    else flux(z, args.a, args.b, args.visc);
   }
   if (args.pro != PRO_LOAD && (args.extra || args.extraf)) {
     // LES additions: jac * tau for a product, the precomputed terms for a flux
     const T es = (args.pro == PRO_PROD) ? from_f64<T>(fc.m.jac[d.m2(k, j)]) : (T)1.0;
-    if (kF && args.extraf)
-      for (int n = lane; n < NX; n += 32) zr[n] = zr[n] + es * (T)args.extraf[base + n];
-    else if (args.extra)
-      for (int n = lane; n < NX; n += 32) zr[n] = zr[n] + es * (T)args.extra[base + n];
+    if (kF && args.extraf) add(z, args.extraf, es);
+    else if (args.extra) add(z, args.extra, es);
   }
   // with fuse_flux the same line's flux term (PRO_FLUX of a2 against b2, and
   // its LES addition) goes through a second transform in the same warp
   const bool fuse = args.fuse_flux != 0;
   V *z2 = smem_c + (size_t)(kWarpsPerBlock + warp) * fstride<E>(M);
   if (fuse) {
-    T *zr2 = reinterpret_cast<T *>(z2);
-    const bool fin2 = kF && args.a2f != nullptr;
-    flux_line<T>([&](int n, T v) { zr2[n] = v; }, fc, k, j, base, lane, fin2, args.a2, args.b2, args.a2f, args.b2f, args.visc2);
-    if (kF && args.extraf2)
-      for (int n = lane; n < NX; n += 32) zr2[n] = zr2[n] + (T)1.0 * (T)args.extraf2[base + n];
-    else if (args.extra2)
-      for (int n = lane; n < NX; n += 32) zr2[n] = zr2[n] + (T)1.0 * (T)args.extra2[base + n];
+    if (kF && args.a2f) flux(z2, args.a2f, args.b2f, args.visc2);
+    else flux(z2, args.a2, args.b2, args.visc2);
+    if (kF && args.extraf2) add(z2, args.extraf2, (T)1.0);
+    else if (args.extra2) add(z2, args.extra2, (T)1.0);
   }
   __syncwarp();
   dif_fft_any<E>(z, M, tw_m<T>(fc), false, lane);
@@ -364,11 +440,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
   const T h = (T)0.5;
   const int NKX = d.NKX;
   const V *twn = tw_n<T>(fc);
-  for (int kk = lane; kk <= d.NX2P; kk += 32) {
-    if (kk > NKX) {
-      if (args.epi == EPI_STORE || args.zero_hi) dst[kk] = cplx_t{0.0, 0.0};
-      continue;
-    }
+  auto emit = [&](int kk, cplx_t o) {
     const int ik = fslot<E>(kk & (M - 1), fc.logM), im = fslot<E>((M - kk) & (M - 1), fc.logM);
     const V w = twn[kk];
     auto split = [&](const V *zz, T &tr, T &ti) {
@@ -384,7 +456,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
       // dst -= i kx X, then dst += X2: the two launches' FP64 updates in order
       T tr2, ti2;
       split(z2, tr2, ti2);
-      const cplx_t o = dst[kk];
       if constexpr (kF) {
         const T kv = from_f64<T>(fc.kx[kk]);
         const cplx_t o1{o.re - f2d_bits((float)(T(0) * tr - kv * ti)), o.im - f2d_bits((float)(T(0) * ti + kv * tr))};
@@ -394,12 +465,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
         const cplx_t o1{o.re - (0.0 * xr - kv * xi), o.im - (0.0 * xi + kv * xr)};
         dst[kk] = cplx_t{o1.re + (double)tr2, o1.im + (double)ti2};
       }
-      continue;
+      return;
     }
     if constexpr (kF) {
       // the FP32 result enters the FP64 field with one exact widening and
       // one FP64 add per component
-      const cplx_t o = (args.epi == EPI_STORE) ? cplx_t{0.0, 0.0} : dst[kk];
       if (args.epi == EPI_STORE) {
         dst[kk] = cplx_t{f2d_bits((float)tr), f2d_bits((float)ti)};
       } else if (args.epi == EPI_ADD) {
@@ -408,22 +478,32 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
         const T kv = from_f64<T>(fc.kx[kk]);
         dst[kk] = cplx_t{o.re - f2d_bits((float)(T(0) * tr - kv * ti)), o.im - f2d_bits((float)(T(0) * ti + kv * tr))};
       }
-      continue;
+      return;
     } else {
     const double xr = (double)tr, xi = (double)ti;
     if (args.epi == EPI_STORE) {
       dst[kk] = cplx_t{xr, xi};
     } else if (args.epi == EPI_ADD) {
-      const cplx_t o = dst[kk];
       dst[kk] = cplx_t{o.re + xr, o.im + xi};
     } else {
       // CF = CF - CIKXP*CS with CIKXP = (0, kx)
       const double kv = fc.kx[kk];
-      const cplx_t o = dst[kk];
       dst[kk] = cplx_t{o.re - (0.0 * xr - kv * xi), o.im - (0.0 * xi + kv * xr)};
     }
     }
+  };
+  constexpr int UE = 3;
+  for (int k0 = lane; k0 <= NKX; k0 += 32 * UE) {
+    cplx_t o[UE];
+#pragma unroll
+    for (int u = 0; u < UE; ++u)
+      o[u] = (args.epi != EPI_STORE && k0 + 32 * u <= NKX) ? dst[k0 + 32 * u] : cplx_t{0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < UE; ++u)
+      if (k0 + 32 * u <= NKX) emit(k0 + 32 * u, o[u]);
   }
+  if (args.epi == EPI_STORE || args.zero_hi)
+    for (int kk = NKX + 1 + lane; kk <= d.NX2P; kk += 32) dst[kk] = cplx_t{0.0, 0.0};
 }
 
 template <typename T, int E>
@@ -444,27 +524,43 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_c2r(FftConst fc, C2rArg
   V *z = smem_c + (size_t)warp * fstride<E>(M);
   const cplx_t *src = args.src + d.ic(0, k, j);
   const cplx_t *src2 = args.src2 ? args.src2 + d.ic(0, k, j) : nullptr;
-  auto X = [&](int kk) -> V {
-    if (kk > NKX || kk >= M) return Cx<T>::make(T(0.0), T(0.0));
-    cplx_t v = src[kk];
-    if (src2) {
-      const cplx_t w = src2[kk];
-      v.re = v.re + args.scale2 * w.re;
-      v.im = v.im + args.scale2 * w.im;
-    }
-    if (args.ik) {  // CIKXP * v
-      const double kv = fc.kx[kk], re = v.re;
-      v.re = -(kv * v.im);
-      v.im = kv * re;
-    }
-    if (kk == 0) v.im = 0.0;
-    return Cx<T>::make(from_f64<T>(v.re), from_f64<T>(v.im));
-  };
   // merge: Z'[k] = (X_k + conj X_{M-k}) + i (X_k - conj X_{M-k}) W^{-k}.
   // The spectrum is staged in z first, so that each mode's prologue (FP64
   // loads, the scale2 combination, the split into T) runs once; then each
   // lane merges the pair (k, M-k) in place (X_M = 0: k = 0 pairs with zero).
-  for (int kk = lane; kk < M; kk += 32) z[kk] = X(kk);
+  // Loads go out four modes a lane at a time, before any of them is used: a
+  // load a turn had 16 KB an SM on the way, and 3 TB/s is what that gives.
+  constexpr int U = (E > 0 && E < 4) ? E : 4;
+  for (int k0 = lane; k0 < M; k0 += 32 * U) {
+    cplx_t v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = (k0 + 32 * u <= NKX) ? src[k0 + 32 * u] : cplx_t{0.0, 0.0};
+    if (src2) {
+      cplx_t w[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) w[u] = (k0 + 32 * u <= NKX) ? src2[k0 + 32 * u] : cplx_t{0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        v[u].re = fma(args.scale2, w[u].re, v[u].re);
+        v[u].im = fma(args.scale2, w[u].im, v[u].im);
+      }
+    }
+    if (args.ik) {  // CIKXP * v
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const double kv = (k0 + 32 * u <= NKX) ? fc.kx[k0 + 32 * u] : 0.0, re = v[u].re;
+        v[u].re = -(kv * v[u].im);
+        v[u].im = kv * re;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int kk = k0 + 32 * u;
+      if (kk >= M) break;
+      if (kk == 0) v[u].im = 0.0;
+      z[kk] = (kk <= NKX) ? Cx<T>::make(from_f64<T>(v[u].re), from_f64<T>(v[u].im)) : Cx<T>::make(T(0.0), T(0.0));
+    }
+  }
   __syncwarp();
   const V *twn = tw_n<T>(fc);
   auto merge = [&](V a, V b, V w) {
@@ -481,35 +577,35 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_c2r(FftConst fc, C2rArg
   }
   __syncwarp();
   dif_fft_any<E>(z, M, tw_m<T>(fc), true, lane);
-  const T *zr = reinterpret_cast<const T *>(z);
   double *dst = args.dst ? args.dst + d.ip(0, k, j) : nullptr;
   float *dstf = args.dstf ? args.dstf + d.ip(0, k, j) : nullptr;
-  const int NX = d.NX;
   if constexpr (std::is_same_v<T, FF>) {
     if (args.dstlo) {
       // float-float planes: the high part is also the field's FP32 copy
       float *dlo = args.dstlo + d.ip(0, k, j);
-      for (int n = lane; n < NX + 2; n += 32) {
-        FF v(0.0f, 0.0f);
-        if (n < NX) v = zr[2 * fslot<E>(n >> 1, fc.logM) + (n & 1)];
-        dstf[n] = v.hi;
-        dlo[n] = v.lo;
+      for (int m = lane; m <= M; m += 32) {
+        const V v = (m < M) ? z[fslot<E>(m, fc.logM)] : Cx<T>::make(T(0.0), T(0.0));
+        *reinterpret_cast<float2 *>(dstf + 2 * m) = make_float2(v.x.hi, v.y.hi);
+        *reinterpret_cast<float2 *>(dlo + 2 * m) = make_float2(v.x.lo, v.y.lo);
       }
       return;
     }
   }
-  for (int n = lane; n < NX + 2; n += 32) {
-    T v = T(0.0);
-    if (n < NX) {
-      const int m = n >> 1;
-      v = zr[2 * fslot<E>(m, fc.logM) + (n & 1)];
-    }
+  // two points at a time; the last pair is the padding x = NX, NX + 1
+  for (int m = lane; m <= M; m += 32) {
+    const V v = (m < M) ? z[fslot<E>(m, fc.logM)] : Cx<T>::make(T(0.0), T(0.0));
     if constexpr (sizeof(T) == 4) {
-      if (dst) dst[n] = f2d_bits((float)v);
-      if (dstf) dstf[n] = (float)v;
+      if (dst) {
+        dst[2 * m] = f2d_bits((float)v.x);
+        dst[2 * m + 1] = f2d_bits((float)v.y);
+      }
+      if (dstf) *reinterpret_cast<float2 *>(dstf + 2 * m) = make_float2((float)v.x, (float)v.y);
     } else {
-      if (dst) dst[n] = (double)v;
-      if (dstf) dstf[n] = d2f_bits((double)v);
+      if (dst) {
+        dst[2 * m] = (double)v.x;
+        dst[2 * m + 1] = (double)v.y;
+      }
+      if (dstf) *reinterpret_cast<float2 *>(dstf + 2 * m) = make_float2(d2f_bits((double)v.x), d2f_bits((double)v.y));
     }
   }
 }
@@ -672,16 +768,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_r2c64(FftConst fc, R2cA
       if (args.pro == PRO_PROD)
         for (int n = lane; n < NX; n += 32) at(zw, l, n) = jac * args.a[base + n] * args.b[base + n];
       else
-        flux_line<double>([&](int n, double v) { at(zw, l, n) = v; }, fc, k, j, base, lane, false, args.a, args.b,
-                          args.af, args.bf, args.visc);
+        flux_line([&](int n, double v) { at(zw, l, n) = v; }, fc, k, j, base, lane, args.a, args.b, args.visc);
       if (args.extra) {
         // LES additions: jac * tau for a product, the precomputed terms for a flux
         const double es = (args.pro == PRO_PROD) ? jac : 1.0;
         for (int n = lane; n < NX; n += 32) at(zw, l, n) += es * args.extra[base + n];
       }
       if (args.fuse_flux) {
-        flux_line<double>([&](int n, double v) { at(zw2, l, n) = v; }, fc, k, j, base, lane, false, args.a2, args.b2,
-                          args.a2f, args.b2f, args.visc2);
+        flux_line([&](int n, double v) { at(zw2, l, n) = v; }, fc, k, j, base, lane, args.a2, args.b2, args.visc2);
         if (args.extra2)
           for (int n = lane; n < NX; n += 32) at(zw2, l, n) += args.extra2[base + n];
       }
@@ -844,6 +938,13 @@ bool launch64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs 
 // and flux transforms, 13.9 -> 11.7 ms a step); in the float-float ones its
 // extra registers cost more than the shared-memory passes it saves, so they
 // keep the loop.
+// What then bounds the FP32 ones is the loads on their way: with one a turn of
+// each loop an SM waits on 16 KB at 3 TB/s.  So points are loaded two at a time
+// and several pairs, or four modes, before any is used.  512 x 385 x 257, a
+// step: forward 8.81 -> 7.84 ms, inverse 5.91 -> 4.95 (six modes at a time
+// 5.55, at the cost of resident blocks); 128 x 129 x 97 0.63 -> 0.56 and 0.66 ->
+// 0.60; 64 x 65 x 65 0.243 -> 0.233 and 0.401 -> 0.388; the float-float
+// inverse of 256 x 193 x 129 2.18 -> 2.02.
 template <typename T>
 void run_r2c(dim3 grid, size_t smem, cudaStream_t s, const FftConst &fc, const R2cArgs &a) {
   const unsigned nt = 32 * kWarpsPerBlock;

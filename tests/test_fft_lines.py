@@ -45,3 +45,30 @@ def test_transforms_match_numpy(nx, lines):
 def test_line_counts_about_the_packing_rule(nx, lines):
     """Both forms on either side of the line count that chooses between them."""
     test_transforms_match_numpy(nx, lines)
+
+
+@pytest.mark.parametrize("nx", [64, 128, 256, 512, 1024])
+@pytest.mark.parametrize("ff", [1, 2])
+def test_mixed_step_at_every_transform_size(nx, ff):
+    """A mixed-path step, straight and sheared, against the FP64 oracle at the
+    mixed path's bar: the transforms' loads in batches at each size."""
+    from ekcases import rel_l2, sheared_case, small_case
+    from ekman_bl_gb300.duct import DuctSolver, metrics_from_grid
+    from ekman_bl_gb300.params import EK_MG_STOP_RESIDUAL
+    from oracle import ekref
+    p, xp, yp, st = (sheared_case if nx in (128, 512) else small_case)(nx=nx)
+    p.mg_stop, p.mg_tol, p.mg_maxcy = EK_MG_STOP_RESIDUAL, 1e-10, 200
+    q = type(p).from_buffer_copy(p)
+    q.mg_maxcy, q.mg_fast, q.fft_fp32, q.ff_arith = 60, 1, 1, ff
+    m = metrics_from_grid(p, xp, yp)
+    g, o = DuctSolver(q, m), ekref.Oracle(p, m)
+    try:
+        g.upload(*st)
+        o.upload(*st)
+        g.step(1)
+        o.step(1)
+        for name, x, y in zip(("CU1", "CU2", "CU3", "CTH"), *[[v[i] for i in (0, 1, 2, 4)] for v in (g.download(), o.download())]):
+            assert rel_l2(x, y) < 1e-5, name
+    finally:
+        g.close()
+        o.close()
