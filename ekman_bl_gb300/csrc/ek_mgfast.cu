@@ -52,11 +52,55 @@ struct FastDev {
   double *red;             // 6 per problem: |b|^2, |r|^2, two unused, meas
   int *done, *cycles, *alldone;
   int *iter;               // corrections applied so far
+  int *count;              // residual blocks finished (f_check)
   double tol;
 };
 
 __device__ __forceinline__ float &E(const LvF &L, int P, int i, int j, int p) {
   return L.e[((size_t)j * (L.nx + 2) + i) * P + p];
+}
+
+// Decide per problem after a residual; iter = corrections applied so far
+// (the device counter plus incr).  A problem within the tolerance is done
+// (1); at iter = maxit the rest stop (2); when none is left, alldone.  In a
+// captured step graph the block also sets the condition of the while-node
+// that repeats the correction cycle: 1 while any problem is active.
+struct CheckF {
+  int on, maxit, incr, use_cond;
+  cudaGraphConditionalHandle cond;
+};
+// All threads of one block, after every block's sums have reached g.red.
+__device__ __forceinline__ void f_check(const FastDev &g, const CheckF &ck, int tid, int nt) {
+  __shared__ int active;
+  const int iter = *g.iter + ck.incr;
+  const bool last = iter >= ck.maxit;
+  if (tid == 0) active = 0;
+  __syncthreads();
+  for (int p = tid; p < g.P; p += nt) {
+    if (g.done[p]) continue;
+    g.cycles[p] = iter;
+    const double bn = sqrt(__ldcg(&g.red[6 * p]));
+    const double meas = (bn > 0.0) ? sqrt(__ldcg(&g.red[6 * p + 1])) / bn : 0.0;
+    const bool conv = meas <= g.tol;
+    g.red[6 * p + 4] = meas;
+    for (int k = 0; k < 4; ++k) g.red[6 * p + k] = 0.0;
+    if (conv) g.done[p] = 1;
+    else if (last) g.done[p] = 2;
+    else atomicAdd(&active, 1);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    *g.iter = iter;
+    if (active == 0) *g.alldone = 1;
+    if (ck.use_cond) cudaGraphSetConditional(ck.cond, active == 0 ? 0u : 1u);
+  }
+}
+__global__ void k_f_check(FastDev g, CheckF ck) {
+  if (*g.alldone) {
+    if (ck.use_cond && threadIdx.x == 0) cudaGraphSetConditional(ck.cond, 0u);
+    return;
+  }
+  f_check(g, ck, (int)threadIdx.x, (int)blockDim.x);
 }
 
 // r = b - A phi at the finest level in float-float (about 48 bits, on the
@@ -67,11 +111,22 @@ __device__ __forceinline__ float &E(const LvF &L, int P, int i, int j, int p) {
 // buffer cycles[p] & 1 (corrections applied so far).  Block row j = 1..ny,
 // lanes over 32 problems; each warp walks a contiguous run of i with the
 // values at i-1, i, i+1 of row j kept in registers.
+// On a small grid the time is that of one run, about 1.5 us a point of
+// dependent float-float operations, so a row is cut into gridDim.z blocks'
+// runs while that fills the SMs (resid_blocks), and with ck.on the last block
+// to finish decides per problem, which saves a launch.  64 x 65 x 65, residual
+// and decision: 15.4 + 4.5 us -> 12.9.  A grid of several waves
+// leaves the decision to k_f_check: there each block's wait for its sums to
+// be visible cost more, 277 us -> 285 against 4 on 512 x 385 x 257.
 constexpr int kRY = 8;
 // (at most 64 registers: four blocks an SM; its loads need the warps)
 template <bool UPDATE, bool ORTH>
-__global__ void __launch_bounds__(32 * kRY, 4) k_f_resid_ff(FastDev g) {
-  if (*g.alldone) return;
+__global__ void __launch_bounds__(32 * kRY, 4) k_f_resid_ff(FastDev g, CheckF ck) {
+  if (*g.alldone) {
+    if (ck.on && ck.use_cond && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0)
+      cudaGraphSetConditional(ck.cond, 0u);
+    return;
+  }
   const int P = g.P;
   const int p = blockIdx.x * 32 + threadIdx.x;
   const int ty = threadIdx.y;
@@ -93,8 +148,8 @@ __global__ void __launch_bounds__(32 * kRY, 4) k_f_resid_ff(FastDev g) {
       if (UPDATE) v = v + FF(ef[q], 0.f);
       return v;
     };
-    const int per = (nx + kRY - 1) / kRY;
-    const int i0 = 1 + ty * per, i1 = min(nx, i0 + per - 1);
+    const int runs = kRY * (int)gridDim.z, per = (nx + runs - 1) / runs;
+    const int i0 = 1 + ((int)blockIdx.z * kRY + ty) * per, i1 = min(nx, i0 + per - 1);
     const size_t row = (size_t)j * (nx + 2) * P + p;
     FF wm, wc;
     if (i0 <= i1) {
@@ -153,6 +208,17 @@ __global__ void __launch_bounds__(32 * kRY, 4) k_f_resid_ff(FastDev g) {
     atomicAdd(&g.red[6 * p], (double)sb);
     atomicAdd(&g.red[6 * p + 1], (double)sr);
   }
+  if (!ck.on) return;
+  __shared__ int mine;
+  __threadfence();  // the sums before the count
+  __syncthreads();
+  const int tid = ty * 32 + (int)threadIdx.x;
+  if (tid == 0) mine = atomicAdd(g.count, 1);
+  __syncthreads();
+  if (mine != (int)(gridDim.x * gridDim.y * gridDim.z) - 1) return;
+  __threadfence();
+  if (tid == 0) *g.count = 0;
+  f_check(g, ck, tid, 32 * kRY);
 }
 
 // Learned initial guess: after k_f_resid_ff on the unscaled guess g
@@ -209,41 +275,6 @@ __global__ void k_f_split(const double *b, float *bh, float *bl, size_t n) {
     const FF v(b[t]);
     bh[t] = v.hi;
     bl[t] = v.lo;
-  }
-}
-
-// Decide per problem after a residual; iter = corrections applied so far
-// (the device counter plus incr).  A problem within the tolerance is done
-// (1); at iter = maxit the rest stop (2); when none is left, alldone.  In a
-// captured step graph the block also sets the condition of the while-node
-// that repeats the correction cycle: 1 while any problem is active.
-__global__ void k_f_check(FastDev g, int maxit, int incr, cudaGraphConditionalHandle cond, int use_cond) {
-  if (*g.alldone) {
-    if (use_cond && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
-    return;
-  }
-  __shared__ int active;
-  const int iter = *g.iter + incr;
-  const bool last = iter >= maxit;
-  if (threadIdx.x == 0) active = 0;
-  __syncthreads();
-  for (int p = threadIdx.x; p < g.P; p += blockDim.x) {
-    if (g.done[p]) continue;
-    g.cycles[p] = iter;
-    const double bn = sqrt(g.red[6 * p]);
-    const double meas = (bn > 0.0) ? sqrt(g.red[6 * p + 1]) / bn : 0.0;
-    const bool conv = meas <= g.tol;
-    g.red[6 * p + 4] = meas;
-    for (int k = 0; k < 4; ++k) g.red[6 * p + k] = 0.0;
-    if (conv) g.done[p] = 1;
-    else if (last) g.done[p] = 2;
-    else atomicAdd(&active, 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *g.iter = iter;
-    if (active == 0) *g.alldone = 1;
-    if (use_cond) cudaGraphSetConditional(cond, active == 0 ? 0u : 1u);
   }
 }
 
@@ -1645,6 +1676,7 @@ FastDev make_fastdev(Ctx &c, int nprob, const double *kx2_dev) {
   g.cycles = w.cycles;
   g.alldone = w.alldone;
   g.iter = w.iter;
+  g.count = w.flags + 2 * w.pmax + 2;
   g.tol = c.p.mg_tol;
   return g;
 }
@@ -1695,14 +1727,23 @@ int tail_level(const MgPlan &PL, int nprob) {
   return top;
 }
 
-void launch_resid_ff(const FastDev &g, bool update, unsigned pch, cudaStream_t s) {
-  const dim3 grid(pch, (unsigned)g.nfy), blk(32, kRY);
+// Blocks resident at once
+constexpr unsigned kResidWave = 4u * 152u;
+// A row's blocks: enough to give every SM its four, of runs of two points and
+// more.  (64 x 65 x 65: 2 x 65 blocks of nine-point runs become 2 x 65 x 4 of
+// three-point ones.)
+unsigned resid_blocks(const FastDev &g, unsigned pch) {
+  const unsigned fill = kResidWave / (pch * (unsigned)g.nfy), most = (unsigned)g.nfx / (2 * kRY);
+  return std::max(1u, std::min(fill, most));
+}
+void launch_resid_ff(const FastDev &g, bool update, unsigned pch, const CheckF &ck, cudaStream_t s) {
+  const dim3 grid(pch, (unsigned)g.nfy, resid_blocks(g, pch)), blk(32, kRY);
   if (update) {
-    if (g.orth) k_f_resid_ff<true, true><<<grid, blk, 0, s>>>(g);
-    else k_f_resid_ff<true, false><<<grid, blk, 0, s>>>(g);
+    if (g.orth) k_f_resid_ff<true, true><<<grid, blk, 0, s>>>(g, ck);
+    else k_f_resid_ff<true, false><<<grid, blk, 0, s>>>(g, ck);
   } else {
-    if (g.orth) k_f_resid_ff<false, true><<<grid, blk, 0, s>>>(g);
-    else k_f_resid_ff<false, false><<<grid, blk, 0, s>>>(g);
+    if (g.orth) k_f_resid_ff<false, true><<<grid, blk, 0, s>>>(g, ck);
+    else k_f_resid_ff<false, false><<<grid, blk, 0, s>>>(g, ck);
   }
 }
 
@@ -1873,7 +1914,7 @@ int mgfast_solve(Ctx &c, int nprob, const double *kx2_dev, const double *kx2_hos
       EK_CUDA(cudaMalloc(&G.alpha, sizeof(float) * nprob));
       G.alpha_cap = nprob;
     }
-    launch_resid_ff(g, false, pch, s);
+    launch_resid_ff(g, false, pch, CheckF{}, s);
     after_launch(c);
     k_f_guess_rb<<<dim3(pch, PL.nfy), dim3(32, kRY), 0, s>>>(g);
     after_launch(c);
@@ -1927,9 +1968,13 @@ int mgfast_solve(Ctx &c, int nprob, const double *kx2_dev, const double *kx2_hos
   auto check = [&](int incr, cudaGraphConditionalHandle cond, int use_cond) {
     // bytes: b (2), r; phi (2), and with the update e and phi' (2)
     KScope ks(c, KC_MG_CHECK, 4.0 * nprob * npt * (incr ? 8.0 : 5.0));
-    launch_resid_ff(g, incr != 0, pch, s);
-    after_launch(c);
-    k_f_check<<<1, 256, 0, s>>>(g, maxit, incr, cond, use_cond);
+    const bool one = pch * (unsigned)g.nfy * resid_blocks(g, pch) <= kResidWave;
+    const CheckF ck{one ? 1 : 0, maxit, incr, use_cond, cond};
+    launch_resid_ff(g, incr != 0, pch, ck, s);
+    if (!one) {
+      after_launch(c);
+      k_f_check<<<1, 256, 0, s>>>(g, ck);
+    }
     after_launch(c);
   };
   // the levels 1..ltop run as one k_f_vtail launch
