@@ -501,10 +501,10 @@ __global__ void __launch_bounds__(64) k_f_xline(FastDev g, int level, int j0, in
 enum { SH_A, SH_B, SH_C, SH_D, SH_YF, SH_VF, SH_WF, SH_YL, SH_VL, SH_WL, SH_S, SH_N };
 // 4-row segments are capped at 48 registers, so that two or three blocks
 // share an SM (their per-thread arrays are half as large)
-template <bool XL, bool ORTH, int LANES, int SEG>
+template <bool XL, bool ORTH, int LANES, int SEG, int REGS = (SEG == 4 ? 48 : 64)>
 // zero_e: the first sweep of a cycle from e = 0 (y-lines only): the
 // neighbouring lines' terms are left out and their stale values unread.
-__global__ void __launch_bounds__(1024) __maxnreg__(SEG == 4 ? 48 : 64) k_f_pline(FastDev g, int level, int l0, int lstep, int mb, int me, int zero_e) {
+__global__ void __launch_bounds__(1024) __maxnreg__(REGS) k_f_pline(FastDev g, int level, int l0, int lstep, int mb, int me, int zero_e) {
   constexpr int kSegMax = SEG;
   if (*g.alldone) return;
   extern __shared__ float sh[];
@@ -1664,6 +1664,9 @@ bool pline_fits(int n, int lanes, int seg) {
   return K <= 128 && K * lanes <= 1024;
 }
 
+// Lines of more rows than this have more than 32 segments of 8: a block of 16
+// problems and 64 registers a thread is then alone on its SM.
+constexpr int kOneBlockRows = 288;
 void launch_pline(const FastDev &g, int l, bool xl, int l0, int lstep, int nline, int n, int lanes, int seg,
                   cudaStream_t s, bool zero_e = false) {
   if (zero_e && xl) throw CudaError("line solve: the zero-neighbour sweep is a y-line sweep");
@@ -1698,6 +1701,8 @@ void launch_pline(const FastDev &g, int l, bool xl, int l0, int lstep, int nline
   } else {
     if (lanes == 32) EK_PLINE(32, 8);
     else if (lanes == 16) EK_PLINE(16, 8);
+    // (three blocks of 8 problems and 43 segments an SM for two: default_lanes)
+    else if (!xl && g.orth && n > kOneBlockRows) k_f_pline<false, true, 8, 8, 56><<<grid, blk, smem, s>>>(g, l, l0, lstep, mb, me, z);
     else EK_PLINE(8, 8);
   }
 #undef EK_PLINE
@@ -1710,7 +1715,18 @@ void launch_pline(const FastDev &g, int l, bool xl, int l0, int lstep, int nline
 // finest x-lines of the largest 213 against 238, of 64 x 225 x 161 21 against
 // 27), and 8 gain 2 to 5% on the finest x-lines alone and lose 10 to 25% on
 // the short ones.
-int default_lanes(int n) { return (pline_segments(n, 8) <= 64) ? 16 : 8; }
+// Beyond 288 rows a block of 16 is alone on its SM, which waits while that block
+// loads, reduces and stores in turn; blocks of 8 share it, three of them for
+// the y-lines of an orthogonal grid at 56 registers (at 64 two; shorter lines
+// and the sheared kernel, with more to hold, are slower at 56).  A sweep,
+// 16 problems against 8: 385 rows of 512 x 385 x 257 314 -> 287 us, 321 rows of
+// 128 x 321 x 193 57.6 -> 52.2, x-lines of 321 of a sheared 256 x 65 x 321 49.5 ->
+// 42.0; sheared y-lines 414 and 405, 74.0 and 75.5, so these keep 16.  Fewer
+// blocks than SMs keep 16 as well (32 x 385 x 129: 20.7 against 24.8).
+int default_lanes(const FastDev &g, bool xl, int n, int nline) {
+  if (pline_segments(n, 8) > 64) return 8;
+  return n > kOneBlockRows && (xl || g.orth) && (long)nline * ((g.P + 15) / 16) > 152 ? 8 : 16;
+}
 
 FastDev make_fastdev(Ctx &c, int nprob, const double *kx2_dev) {
   const MgPlan &PL = c.mg;
@@ -1991,7 +2007,7 @@ int mgfast_solve(Ctx &c, int nprob, const double *kx2_dev, const double *kx2_hos
 
   // one partitioned line launch, in the layout tuned for (level, direction)
   auto pline = [&](int l, bool xl, int l0, int lstep, int nline, int n, bool zero_e) {
-    int lanes = default_lanes(n), seg = 8;
+    int lanes = default_lanes(g, xl, n, nline), seg = 8;
     const std::vector<int> &tl = xl ? PL.lanes_x : PL.lanes_y;
     const std::vector<int> &ts = xl ? PL.seg_x : PL.seg_y;
     if (l < (int)tl.size() && tl[l] > 0) lanes = tl[l];
