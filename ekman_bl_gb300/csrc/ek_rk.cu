@@ -842,6 +842,116 @@ __global__ void __launch_bounds__(32 * kLesWarps) k_adi_les_tile(AdiArgs a) {
   }
 }
 
+// The y sweep of k_adi_les_tile with one thread a system, kLesChunk rows'
+// loads at a time: the same operations on the same values.  With the GPU filled
+// by systems alone the tile's exchange through shared memory costs more than
+// the latency it hides, so this form takes a sweep whose blocks (seven of 72
+// registers an SM) fill the waves they run in to 85%.  The four fields' sweeps
+// of a step, tile against this: 0.96 of a wave (512 x 385 x 257) 19.1 and 17.2
+// ms, 2.88 waves (1024 x 513 x 385) 75 and 71; 0.72 (512 x 193 x 193) 7.4 and
+// 7.7, 1.44 (1024 x 257 x 193) 19.3 and 20.0, 0.24 (256 x 193 x 129) 3.2 and 6.4.
+// (The z sweep: 15.2 and 17.3 at 512 x 385 x 257, 60 and 58 at 1024 x 513 x 385;
+// the tile at all sizes.)
+inline bool les_one_thread(int nx, int lines) {
+  const int blocks = (nx + 127) / 128 * lines, wave = 7 * 152;
+  return 100L * blocks >= 85L * ((blocks + wave - 1) / wave) * wave;
+}
+__global__ void __launch_bounds__(128) k_adi_les_y(AdiArgs a) {
+  const Dims &d = a.d;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int line = a.zs + (int)blockIdx.y;
+  if (i >= d.NX) return;
+  const int nrow = d.NY2, r0 = a.js, r1 = a.je;
+  const int n2 = d.LDM * (d.NY + 3);
+  const size_t sX = d.LDX, sA = (size_t)d.LDX * d.NZ2;
+  const float *nut = a.nutf;
+  const double *po = a.phi_old;
+  float2 *gout = reinterpret_cast<float2 *>(a.out);
+  float2 *sb = reinterpret_cast<float2 *>(a.scr_b), *su = reinterpret_cast<float2 *>(a.scr_u);
+  const size_t c0 = d.ip(i, line, 0);
+  constexpr int CH = kLesChunk, CB = kAdiChunk;
+  FF rBp(1.0f, 0.0f), gp(0.0f, 0.0f), Up(0.0f, 0.0f);
+  for (int rc = 0; rc < nrow; rc += CH) {
+    FF Lv[CH], Dv[CH], Uv[CH], Vv[CH];
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      const int r = rc + u;
+      const size_t c = c0 + (size_t)r * sA;
+      FF L(0.0f, 0.0f), D(1.0f, 0.0f), U(0.0f, 0.0f), V(0.0f, 0.0f);
+      if (r >= r0 && r <= r1) {
+        const float2 *t = a.ftab + (line + r * d.LDM);
+        const float nu0 = nut[c], nap = nut[c + sA], nam = nut[c - sA], nxp = nut[c + sX], nxm = nut[c - sX];
+        const FF f0(po[c]), fxp(po[c + sX]), fxm(po[c - sX]);
+        const FF v = FF(0.5f * a.Sf[c], 0.5f * 0.0f) + ff2(t[0]) * f0 + ff2(t[n2]) * fxp + ff2(t[2 * n2]) * fxm;
+        const FF tp = ff2(t[9 * n2]) * (ff1(nxp) + ff1(nu0)), tm = ff2(t[10 * n2]) * (ff1(nu0) + ff1(nxm));
+        V = v + tp * (fxp - f0) - tm * (f0 - fxm);
+        const FF slo = ff1(nu0) + ff1(nam), sup = ff1(nu0) + ff1(nap);
+        const FF ml = ff2(t[7 * n2]), mu = ff2(t[8 * n2]);
+        L = ff2(t[4 * n2]) - ml * slo;
+        U = ff2(t[5 * n2]) - mu * sup;
+        D = ff2(t[6 * n2]) + mu * sup + ml * slo;
+      }
+      if (r < nrow)
+        for (int b = 0; b < a.bc.n; ++b) {
+          const BcRow &br = a.bc.r[b];
+          if (br.row != r) continue;
+          L = FF(br.l);
+          D = FF(br.dg);
+          U = FF(br.u);
+          if (br.kind == 0) V = FF(br.val);
+          else if (br.kind == 1) V = FF(po[d.ip(i, line, br.src)]);
+          else V = FF(br.val * a.bcw[br.src + line]);
+        }
+      Lv[u] = L;
+      Dv[u] = D;
+      Uv[u] = U;
+      Vv[u] = V;
+    }
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      const int r = rc + u;
+      if (r >= nrow) break;
+      const size_t c = c0 + (size_t)r * sA;
+      FF B = Dv[u], g = Vv[u];
+      if (r > 0) {
+        const FF am = -(Lv[u] * rBp);
+        B = Dv[u] + am * Up;
+        g = Vv[u] + am * gp;
+      }
+      const FF rB = ff_rcp(B);
+      gout[c] = make_float2(g.hi, g.lo);
+      sb[c] = make_float2(rB.hi, rB.lo);
+      su[c] = make_float2(Uv[u].hi, Uv[u].lo);
+      rBp = rB;
+      gp = g;
+      Up = Uv[u];
+    }
+  }
+  FF x = gp * rBp;
+  auto put = [&](int r) {
+    const FF y = ff_round53(x);
+    gout[c0 + (size_t)r * sA] = make_float2(y.hi, y.lo);
+  };
+  put(nrow - 1);
+  for (int rc = nrow - 2; rc >= 0; rc -= CB) {
+    float2 gv[CB], uv[CB], bv[CB];
+#pragma unroll
+    for (int u = 0; u < CB; ++u)
+      if (rc - u >= 0) {
+        const size_t c = c0 + (size_t)(rc - u) * sA;
+        gv[u] = gout[c];
+        uv[u] = su[c];
+        bv[u] = sb[c];
+      }
+#pragma unroll
+    for (int u = 0; u < CB; ++u)
+      if (rc - u >= 0) {
+        x = (ff2(gv[u]) - ff2(uv[u]) * x) * ff2(bv[u]);
+        put(rc - u);
+      }
+  }
+}
+
 // CN-ADI line solves, one thread per system (one x point of one line).
 // y sweep (ZS = false), duct.F90:1640-1739 for U1 (TH 1334-1433, U2
 // 1877-1980, U3 2137-2233): R' = S/2 + J phi + coef d_zeta(G11 d_zeta phi),
@@ -852,7 +962,7 @@ __global__ void __launch_bounds__(32 * kLesWarps) k_adi_les_tile(AdiArgs a) {
 // solved range take the y-sweep values.
 // The thread forms each row's right-hand side from the per-cell weights
 // (k_adi_tab), runs the forward elimination of THOMAS_REAL with the line's
-// host factors (broadcast loads: a block's threads share the line) and parks
+// precomputed factors (broadcast loads: a block's threads share the line) and parks
 // the modified right-hand side in the output, then back-substitutes.  Along
 // y, rows go kAdiChunk at a time: every load of a chunk is issued before the
 // recurrence consumes it, so a thread keeps that many rows' loads in flight
@@ -948,7 +1058,7 @@ __global__ void __launch_bounds__(128) k_adi_seq(AdiArgs a) {
 // k_adi_seq (explicit-increment form) on float-float fields, for the mixed
 // path: the old field, the y-sweep result and the new field are float-float
 // planes and every row runs in float-float arithmetic (about 48 bits) on the
-// FP32 pipe, from the same per-cell weights and host Thomas factors split
+// FP32 pipe, from the same per-cell weights and Thomas factors split
 // into float pairs; the only FP64 work left is a boundary row's constant.
 template <bool ZS>
 __global__ void __launch_bounds__(128) k_adi_ffs(AdiArgs a) {
@@ -1063,7 +1173,7 @@ __global__ void __launch_bounds__(128) k_adi_ffs(AdiArgs a) {
 // increment d*; the z sweep's base is phi* = phi_old + d* (d* = 0 on the
 // lines the y sweep leaves alone) and its output the total increment
 // phi_new - phi_old, whose FP32 forward transform is added to the spectral
-// state.  The same host Thomas factors and per-cell weights, rounded to
+// state.  The same Thomas factors and per-cell weights, rounded to
 // FP32, drive the elimination.
 template <bool ZS>
 __global__ void __launch_bounds__(128) k_adi_inc(AdiArgs a) {
@@ -2103,7 +2213,8 @@ void launch_adi(Ctx &c, int field, int rk) {
       dim3 grid((d.NX + 127) / 128, a.ze - a.zs + 1), tiles((d.NX + 31) / 32, a.ze - a.zs + 1);
       // algorithmic: read R, the field and NU_T, write the result
       KScope ks(c, KC_ADI_Y, 32.0 * d.NX * d.NY2 * (a.ze - a.zs + 1));
-      if (ff) k_adi_les_tile<false><<<tiles, 32 * kLesWarps, 0, c.stream>>>(a);
+      if (ff && les_one_thread(d.NX, a.ze - a.zs + 1)) k_adi_les_y<<<grid, 128, 0, c.stream>>>(a);
+      else if (ff) k_adi_les_tile<false><<<tiles, 32 * kLesWarps, 0, c.stream>>>(a);
       else if (a.Sf) k_adi_les<false, true><<<grid, 128, 0, c.stream>>>(a);
       else k_adi_les<false, false><<<grid, 128, 0, c.stream>>>(a);
       after_launch(c);

@@ -40,3 +40,10 @@ def test_tiled_line_solves_track_oracle(case, nx, ny2, nz2):
     for name, f in zip(("CU1", "CU2", "CU3", "CTH"), (0, 1, 2, 4)):
         e = rel_l2(a[f], b[f])
         assert np.isfinite(e) and e < 1e-5, (name, e)
+
+
+@pytest.mark.parametrize("nx,ny2,nz2", [(512, 19, 257), (1024, 9, 129)])
+def test_one_thread_a_system_tracks_oracle(nx, ny2, nz2):
+    """Sweeps of enough lines that the float-float y sweep with LES goes one
+    thread a system (rows short of and past whole chunks of 4 and 8)."""
+    test_tiled_line_solves_track_oracle("les", nx, ny2, nz2)
