@@ -872,10 +872,11 @@ __device__ __forceinline__ void f_prolong_y_at(const float *__restrict__ scr, fl
 // coarse rows of it: their stage-1 values and those of the rows around, the e
 // they go to, then the sums, the same as above one by one.  All loads go out
 // together.  Block (32 problems, kProRows coarse rows, every gridDim.z-th
-// eight columns).  512 x 385 x 257, every problem active, finest level: 51 + 124
-// -> 120 us; all transfers of a step: 8.56 -> 7.37 ms, 256 x 193 x 129 2.15 ->
-// 1.74, 128 x 129 x 97 0.94 -> 0.70.
-constexpr int kProRows = 4;
+// eight columns).  All transfers of a step: 512 x 385 x 257 8.56 -> 6.93 ms, 256 x
+// 193 x 129 2.15 -> 1.68, 128 x 129 x 97 0.94 -> 0.65.  Four rows a thread form
+// fewer stage-1 values twice, but hold 51 loads at a time for 27 and leave the
+// SMs fewer warps: 7.38, 1.75 and 0.68.
+constexpr int kProRows = 2;
 __global__ void __launch_bounds__(32 * kRowWarps) k_f_prolong(FastDev g, int level) {
   if (*g.alldone) return;
   const LvF F = g.lv[level - 1], C = g.lv[level - 2];
@@ -885,6 +886,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_f_prolong(FastDev g, int lev
   const int nx = F.nx, ny = F.ny, ncx = C.nx, ncy = C.ny;
   const int r0 = (int)blockIdx.y * kProRows;  // coarse rows r0 + 1 ..
   constexpr int N = kProRows + 3;
+  static_assert(N >= 5, "the first row between takes four stage-1 rows");
   const bool ycoarse = ncy < ny, cubic = ncy >= 4;
   const float *ce = C.e + p;
   float *ef = F.e + p;
