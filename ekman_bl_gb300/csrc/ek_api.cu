@@ -1390,7 +1390,8 @@ int ekgpu_unet_train_step(ek_unet *u, const float *x_dev, const float *t_dev, in
   return unet_guarded(u, [&](ek::UNet &net) {
     if (!x_dev || !t_dev || n < 1 || n > net.max_n || hv < 1 || hv > net.h || wv < 1 || wv > net.w)
       return (int)EK_ERR_ARG;
-    const double l = net.train_step(x_dev, t_dev, n, hv, wv, lr, (cudaStream_t)stream);
+    double l = 0.0;
+    if (!net.train_step(x_dev, t_dev, n, hv, wv, lr, l, (cudaStream_t)stream)) return (int)EK_ERR_TIMEOUT;
     if (loss) *loss = l;
     return (int)EK_OK;
   });
@@ -1401,7 +1402,8 @@ int ekgpu_unet_gradient(ek_unet *u, const float *x_dev, const float *t_dev, int 
   return unet_guarded(u, [&](ek::UNet &net) {
     if (!x_dev || !t_dev || n < 1 || n > net.max_n || hv < 1 || hv > net.h || wv < 1 || wv > net.w)
       return (int)EK_ERR_ARG;
-    const double l = net.forward_backward(x_dev, t_dev, n, hv, wv, y_dev, (cudaStream_t)stream);
+    double l = 0.0;
+    if (!net.forward_backward(x_dev, t_dev, n, hv, wv, y_dev, l, (cudaStream_t)stream)) return (int)EK_ERR_TIMEOUT;
     if (loss) *loss = l;
     if (grad_host)
       EK_CUDA(cudaMemcpy(grad_host, net.grads(), sizeof(float) * net.nparams(), cudaMemcpyDeviceToHost));

@@ -1262,7 +1262,8 @@ UNet::UNet(int cin_, int C_, int max_n_, int h_, int w_) : cin(cin_), C(C_), max
     grad_ = (float *)alloc(sizeof(float) * nparam_, bufs_);
     m_ = (float *)alloc(sizeof(float) * nparam_, bufs_);
     v_ = (float *)alloc(sizeof(float) * nparam_, bufs_);
-    loss_ = (double *)alloc(sizeof(double), bufs_);
+    loss_ = (double *)alloc(2 * sizeof(double), bufs_);
+    tc_err_ = (int *)(loss_ + 1);
     xin_ = (unsigned short *)alloc(img_bytes(max_n, h, w, cin, 2), bufs_);
     for (int l = 0; l < kLevels; ++l) {
       const int hl = h >> l, wl = w >> l;
@@ -1276,7 +1277,6 @@ UNet::UNet(int cin_, int C_, int max_n_, int h_, int w_) : cin(cin_), C(C_), max
       }
     }
     y_ = (float *)alloc(sizeof(float) * (size_t)max_n * h * w, bufs_);
-    tc_err_ = (int *)alloc(sizeof(int), bufs_);
   } catch (...) {
     for (void *p : bufs_) cudaFree(p);
     bufs_.clear();
@@ -1418,7 +1418,8 @@ int UNet::tc_error(cudaStream_t s) {
   return v;
 }
 
-double UNet::forward_backward(const float *x, const float *t, int n, int hv, int wv, float *y, cudaStream_t s) {
+bool UNet::forward_backward(const float *x, const float *t, int n, int hv, int wv, float *y, double &loss,
+                            cudaStream_t s) {
   if (!y) y = y_;
   run_forward(x, n, y, s);
   alloc_grads(n);
@@ -1538,14 +1539,18 @@ double UNet::forward_backward(const float *x, const float *t, int n, int hv, int
   }
   back(1, 0, t_[0], nullptr, gs_[0], gsb_[0], gt_[0], gtb_[0], t_[0], nullptr, nullptr);
   back(0, 0, xin_, nullptr, gt_[0], gtb_[0], nullptr, nullptr, nullptr, nullptr, nullptr);
-  double loss = 0.0;
-  EK_CUDA(cudaMemcpyAsync(&loss, loss_, sizeof(double), cudaMemcpyDeviceToHost, s));
+  struct {
+    double loss;
+    int err;
+  } res = {};
+  EK_CUDA(cudaMemcpyAsync(&res, loss_, sizeof(res), cudaMemcpyDeviceToHost, s));
   EK_CUDA(cudaStreamSynchronize(s));
-  return loss;
+  loss = res.loss;
+  return !(tc_ && res.err);
 }
 
-double UNet::train_step(const float *x, const float *t, int n, int hv, int wv, double lr, cudaStream_t s) {
-  const double loss = forward_backward(x, t, n, hv, wv, nullptr, s);
+bool UNet::train_step(const float *x, const float *t, int n, int hv, int wv, double lr, double &loss, cudaStream_t s) {
+  if (!forward_backward(x, t, n, hv, wv, nullptr, loss, s)) return false;
   ++step_;
   const double b1 = 0.9, b2 = 0.999;
   const double lr_t = lr * std::sqrt(1.0 - std::pow(b2, (double)step_)) / (1.0 - std::pow(b1, (double)step_));
@@ -1553,7 +1558,7 @@ double UNet::train_step(const float *x, const float *t, int n, int hv, int wv, d
   ++launches_;
   const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) throw CudaError(std::string("unet adam: ") + cudaGetErrorString(e));
-  return loss;
+  return true;
 }
 
 }  // namespace ek

@@ -30,9 +30,12 @@ class UNet {
   void forward(const float *x, int n, float *y, cudaStream_t s);
   // Forward, mean-square error against t over the top-left hv x wv pixels
   // of each image, backward; the parameter gradient lands in grads().
-  double forward_backward(const float *x, const float *t, int n, int hv, int wv, float *y, cudaStream_t s);
-  // forward_backward, then one Adam step (lr, beta1 0.9, beta2 0.999, eps 1e-8)
-  double train_step(const float *x, const float *t, int n, int hv, int wv, double lr, cudaStream_t s);
+  // False: a tcgen05 convolution's bounded wait ran out, and loss, prediction
+  // and gradient are not to be used.
+  bool forward_backward(const float *x, const float *t, int n, int hv, int wv, float *y, double &loss, cudaStream_t s);
+  // forward_backward, then one Adam step (lr, beta1 0.9, beta2 0.999, eps
+  // 1e-8); false: as above, and the parameters and the Adam state are as before
+  bool train_step(const float *x, const float *t, int n, int hv, int wv, double lr, double &loss, cudaStream_t s);
   const float *grads() const { return grad_; }
   long launches() const { return launches_; }
   double forward_flops(int n) const;  // 2 x multiply-adds of the convolutions
@@ -58,7 +61,7 @@ class UNet {
   long step_ = 0;
   long launches_ = 0;
   bool tc_ = true;
-  int *tc_err_ = nullptr;
+  int *tc_err_ = nullptr;  // behind *loss_, so that one copy brings both
   // activations (BF16, bordered): xin, t[l], s[l], p[l], u[l], v[l], d[l]
   unsigned short *xin_ = nullptr;
   unsigned short *t_[kLevels] = {}, *s_[kLevels] = {}, *p_[kLevels] = {};
