@@ -1206,6 +1206,20 @@ TcShape tc_shape(const Img &g, int cin, int cout) {
   while (t.ncols < 2 * cout) t.ncols *= 2;
   return t;
 }
+// Whether a layer runs on the tensor-core kernels, forward, input gradient and
+// weight gradient alike: the weight gradient and the input gradient below read
+// the BF16 copy that the input gradient above has written, so a network's
+// passes must not mix k_conv_tc with k_conv_gemm, which writes FP32 alone.
+bool tc_channels(int cin, int cout, int c1) { return cin % 16 == 0 && cout % 16 == 0 && c1 % 16 == 0; }
+// Such a layer must fit k_conv_tc in both directions, and is refused beyond 220
+// KB for 128 + cout rows of 9 cin BF16 values: networks of 16 and 32 channels run
+// (one stage takes at most 170 KB, whatever the image), 48 and 64 need
+// set_tcgen05(0).
+void tc_require(const Img &g, int cin, int cout) {
+  if ((size_t)(tc::kM + cout) * 9 * cin * 2 + 16 > kTcSmem || tc_shape(g, cin, cout).smem() > kTcSmem ||
+      tc_shape(g, cout, cin).smem() > kTcSmem)
+    throw CudaError("unet: tcgen05 tile does not fit in shared memory");
+}
 template <bool DX>
 void launch_tc(const ConvArgs &a, const TcShape &t, int *err, cudaStream_t s) {
   kernel_limits();
@@ -1359,11 +1373,9 @@ void UNet::run_forward(const float *x, int n, float *y, cudaStream_t s) {
     a.y32 = out32;
     a.relu = Ly.relu;
     const long M = (long)n * a.g.H * a.g.W;
-    if (tc_ && !out32 && Ly.cin % 16 == 0 && Ly.c1 % 8 == 0 && Ly.c2 % 8 == 0 && Ly.cout % 16 == 0) {
-      const TcShape t = tc_shape(a.g, Ly.cin, Ly.cout);
-      if ((size_t)(tc::kM + Ly.cout) * 9 * Ly.cin * 2 + 16 > kTcSmem || t.smem() > kTcSmem)
-        throw CudaError("unet: tcgen05 tile does not fit in shared memory");
-      launch_tc<false>(a, t, tc_err_, s);
+    if (tc_ && tc_channels(Ly.cin, Ly.cout, Ly.c1)) {
+      tc_require(a.g, Ly.cin, Ly.cout);
+      launch_tc<false>(a, tc_shape(a.g, Ly.cin, Ly.cout), tc_err_, s);
     } else if (tc_ && out32 && Ly.cout == 1 && !Ly.c2) {
       k_conv_last<<<gsz(M, 256), 256, sizeof(float) * 9 * Ly.cin, s>>>(a);
     } else if (tc_ && !out32 && Ly.cin <= 4 && Ly.cout <= 64 && !Ly.c2) {
@@ -1457,7 +1469,7 @@ bool UNet::forward_backward(const float *x, const float *t, int n, int hv, int w
     a.m2 = m2;
     const long npx = (long)n * a.g.H * a.g.W;
     const long stored = (long)n * (a.g.H + 2) * (a.g.W + 2);
-    const bool mult16 = tc_ && Ly.cin % 16 == 0 && Ly.cout % 16 == 0 && Ly.c1 % 16 == 0;
+    const bool mult16 = tc_ && tc_channels(Ly.cin, Ly.cout, Ly.c1);
     const bool last = tc_ && Ly.cout == 1 && !Ly.c2 && Ly.cin % 8 == 0;
     if (mult16) {
       kernel_limits();
@@ -1501,9 +1513,8 @@ bool UNet::forward_backward(const float *x, const float *t, int n, int hv, int w
     }
     K.check();
     if (!dx1) return;
-    const TcShape t = tc_shape(a.g, Ly.cout, Ly.cin);
-    if (mult16 && t.smem() <= kTcSmem) {
-      launch_tc<true>(a, t, tc_err_, s);
+    if (mult16) {
+      launch_tc<true>(a, tc_shape(a.g, Ly.cout, Ly.cin), tc_err_, s);
     } else if (last) {
       k_dx_last<<<(unsigned)std::min((npx + 63) / 64, 8L * sm_count()), 128, 0, s>>>(a);
     } else {
