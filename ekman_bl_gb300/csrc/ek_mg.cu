@@ -751,11 +751,23 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
 }
 
 constexpr size_t kRelaxSmem = 220 * 1024;
-// k_relax_block takes the sheared grids' levels whose phi fits a block, while
-// the 20 phase launches of a sweep cost more than the FP64 work that stays on
-// one SM a problem
+// k_relax_block takes the sheared grids' levels whose phi fits a block, for
+// batches of at most six waves of the blocks the GPU holds at once (two an SM up
+// to 114 KB, one beyond), or three where more than 196 KB of shared memory leave
+// the SM's L1 too little to keep the coefficients (a wave then takes twice as
+// long). The 20 phase launches of a sweep spread a large batch's FP64 work over
+// all SMs without waves, but cost 5 us each however small the batch. A batch's
+// finest sweeps, block against phases, ms: 129 x 97 with 44 problems 2.8 and 8.9,
+// 1,368 (5 waves) 11.9 and 13.7, 2,052 (7) 16.9 and 15.2; 177 x 129 with 760 (5)
+// 12.4 and 14.4, 1,026 (7) 15.7 and 15.3; 177 x 145 with 456 (3) 12.4 and 13.4,
+// 532 (4) 15.0 and 13.6, 684 (5) 17.7 and 14.5; 161 x 161 with 684 17.6 and 14.7.
+constexpr size_t kSmemSM = 228 * 1024, kSmemKept = 1024;  // of an SM; a block's own share besides
 bool relax_in_block(const MgPlan &PL, const MgLevel &L, int nprob) {
-  return !PL.orth && relax_block_smem(L.nx, L.ny) <= kRelaxSmem;
+  const size_t smem = relax_block_smem(L.nx, L.ny);
+  if (PL.orth || smem > kRelaxSmem) return false;
+  const size_t sm = smem + kSmemKept;
+  const int resident = (2 * sm <= kSmemSM) ? 2 : 1, waves = (sm > 196 * 1024) ? 3 : 6;
+  return nprob <= waves * resident * 152;
 }
 
 unsigned nblk(long n, int bs) {
