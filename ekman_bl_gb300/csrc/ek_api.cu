@@ -979,6 +979,9 @@ int ekgpu_set_metrics(ek_ctx *h, const ek_metrics *m) {
       if (!c.mg_z) c.mg_z = dalloc<double>(c, z.size());
       EK_CUDA(cudaMemcpy(c.mg_z, z.data(), sizeof(double) * z.size(), cudaMemcpyHostToDevice));
     }
+    // the levels that one block of k_coarse holds: level 1, and those above it
+    // while their phi, rhs, 1/c9 and couplings and the scratch fit 96 KB (the
+    // kernel keeps c9 as well)
     const int ncof = P.orth ? 4 : 8;
     P.lc = 1;
     for (int l = 1; l <= P.ngrid; ++l) {

@@ -977,8 +977,11 @@ void mg_null_mean(Ctx &c, double *phi_finest, int nprob, const double *kx2_dev) 
 void mg_exact_attributes() {
   static std::once_flag once;
   std::call_once(once, [] {
-    EK_CUDA(cudaFuncSetAttribute(k_coarse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    EK_CUDA(cudaFuncSetAttribute(k_coarse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    // k_coarse: levels 1..lc take up to 112 KB (96 KB counted without c9), but a
+    // level 1 larger than that is in it whatever its size, up to the most a
+    // block can have
+    EK_CUDA(cudaFuncSetAttribute(k_coarse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemSM - kSmemKept)));
+    EK_CUDA(cudaFuncSetAttribute(k_coarse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemSM - kSmemKept)));
     EK_CUDA(cudaFuncSetAttribute(k_relax_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRelaxSmem));
   });
 }
