@@ -503,9 +503,7 @@ __global__ void k_check_finish(MgDev g, int iter, int last) {
 // Coarse levels 1..lc: one CTA per problem, everything in shared memory.
 struct CoarseLv {
   int nx, ny;
-  // offsets (doubles) into shared memory; rhs and cof hold rhs / c9 and the
-  // couplings / c9, so that an update is one multiply-add a coupling
-  int phi, rhs, inv9, c9, cof;
+  int phi, rhs, inv9, c9, cof;  // offsets (doubles) into shared memory
 };
 struct CoarseArgs {
   MgDev g;
@@ -523,15 +521,18 @@ constexpr int kCoarseThreads = 256;
 // takes: a warp's FP64 instruction holds its quarter of the SM for 64 clocks,
 // however many of its lanes work (measured), so the points are packed over
 // the threads, and while the phase fits four warps that way two lanes share a
-// point's couplings and add their halves.  (One lane a point and the sum and
-// right-hand side scaled last: ten dependent operations, 298 us a launch on
-// 64 x 129 x 97 sheared; now 178.)
+// point's couplings and add their halves.  (One lane a point: ten dependent
+// operations, 298 us a launch on 64 x 129 x 97 sheared; now 187.  With the
+// right-hand side and the couplings divided by c9 beforehand a point takes one
+// operation less, 178 us, but each such quotient is rounded: on grids of one
+// block, solved to convergence, up to four times the error against 64-bit
+// exact solutions.)
 template <bool ORTH>
 __device__ __forceinline__ void c_relax(const CoarseArgs &A, double *sm, int level, int count, int &stale) {
   const CoarseLv &L = A.lv[level - 1];
   const int nx = L.nx, ny = L.ny;
   double *phi = sm + L.phi;
-  const double *rhs = sm + L.rhs, *cf = sm + L.cof;
+  const double *rhs = sm + L.rhs, *cf = sm + L.cof, *inv9 = sm + L.inv9;
   const int npt = nx * ny;
   const int sj = nx + 2;
   const bool onwrite = ORTH && (nx % 4 != 2);
@@ -571,10 +572,12 @@ __device__ __forceinline__ void c_relax(const CoarseArgs &A, double *sm, int lev
             v = v - kk[2 * npt] * ph[g * sj];
             return v - kk[3 * npt] * ph[g * (sj - 1)];
           };
+          const double iv = inv9[pt];
           double v = half ? 0.0 : rhs[pt];
           v = ahead(v, k, sg);
           if (split) v += __shfl_xor_sync(0xffffffffu, v, 1);
           else v = ahead(v, k + H * npt, -1);
+          v = v * iv;
           if (on && !half) {
             *ph = v;
             if (onwrite) {
@@ -608,27 +611,27 @@ __device__ __forceinline__ void c_restrict(const CoarseArgs &A, double *sm, int 
   for (int t = threadIdx.x; t < nx * ny; t += blockDim.x) {
     const int i = 1 + t % nx, j = 1 + t / nx;
     const double *ph = phi + j * sj + i;
-    double s = rhs[t] - cf[t] * ph[1];
+    double s = cf[t] * ph[1];
     if (ORTH) {
-      s = s - cf[npt + t] * ph[sj];
-      s = s - cf[2 * npt + t] * ph[-1];
-      s = s - cf[3 * npt + t] * ph[-sj];
+      s = s + cf[npt + t] * ph[sj];
+      s = s + cf[2 * npt + t] * ph[-1];
+      s = s + cf[3 * npt + t] * ph[-sj];
     } else {
-      s = s - cf[npt + t] * ph[1 + sj];
-      s = s - cf[2 * npt + t] * ph[sj];
-      s = s - cf[3 * npt + t] * ph[sj - 1];
-      s = s - cf[4 * npt + t] * ph[-1];
-      s = s - cf[5 * npt + t] * ph[-1 - sj];
-      s = s - cf[6 * npt + t] * ph[-sj];
-      s = s - cf[7 * npt + t] * ph[1 - sj];
+      s = s + cf[npt + t] * ph[1 + sj];
+      s = s + cf[2 * npt + t] * ph[sj];
+      s = s + cf[3 * npt + t] * ph[sj - 1];
+      s = s + cf[4 * npt + t] * ph[-1];
+      s = s + cf[5 * npt + t] * ph[-1 - sj];
+      s = s + cf[6 * npt + t] * ph[-sj];
+      s = s + cf[7 * npt + t] * ph[1 - sj];
     }
-    scr[j * sj + i] = c9[t] * (s - ph[0]);
+    s = s + c9[t] * ph[0];
+    scr[j * sj + i] = rhs[t] - s;
   }
   __syncthreads();
   const int ix = (ncx == nx) ? 0 : 1, jy = (ncy == ny) ? 0 : 1;
   double *phic = sm + C.phi;
   double *rhsc = sm + C.rhs;
-  const double *iv = sm + C.inv9;
   for (int t = threadIdx.x; t < (ncx + 2) * (ncy + 2); t += blockDim.x) phic[t] = 0.0;
   for (int t = threadIdx.x; t < ncx * ncy; t += blockDim.x) {
     const int ic = 1 + t % ncx, jc = 1 + t / ncx;
@@ -646,7 +649,7 @@ __device__ __forceinline__ void c_restrict(const CoarseArgs &A, double *sm, int 
     }
     auto R = [&](int a, int b) { return scr[b * sj + a]; };
     rhsc[t] = (R(im1, jm1) + R(ip1, jm1) + R(im1, jp1) + R(ip1, jp1) +
-               2. * (R(im1, j) + R(ip1, j) + R(i, jm1) + R(i, jp1)) + 4. * R(i, j)) * .0625 * iv[t];
+               2. * (R(im1, j) + R(ip1, j) + R(i, jm1) + R(i, jp1)) + 4. * R(i, j)) * .0625;
   }
   __syncthreads();
 }
@@ -708,7 +711,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
   const int p = blockIdx.x;
   if (*g.alldone || g.done[p]) return;
   const int P = g.P;
-  // load every coarse level (phi with ghosts, 1/c9, c9, rhs / c9, couplings / c9)
+  // load every coarse level (phi with ghosts, rhs, 1/c9, c9, couplings)
   const double kx2 = g.kx2[p];
   for (int l = 1; l <= g.lc; ++l) {
     const CoarseLv &L = A.lv[l - 1];
@@ -718,14 +721,13 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
     for (int t = threadIdx.x; t < nph; t += kCoarseThreads) sm[L.phi + t] = G.phi[(size_t)t * P + p];
 #pragma unroll 2
     for (int t = threadIdx.x; t < npt; t += kCoarseThreads) {
-      const double iv = G.inv9[(size_t)t * P + p];
-      sm[L.rhs + t] = G.rhs[(size_t)t * P + p] * iv;
-      sm[L.inv9 + t] = iv;
+      sm[L.rhs + t] = G.rhs[(size_t)t * P + p];
+      sm[L.inv9 + t] = G.inv9[(size_t)t * P + p];
       sm[L.c9 + t] = ((-kx2 * G.cof[(size_t)10 * npt + t]) - G.cof[(size_t)8 * npt + t]) + G.cof[(size_t)9 * npt + t];
       // c1, c3, c5, c7 or c1..c8
 #pragma unroll
       for (int q = 0; q < (ORTH ? 4 : 8); ++q)
-        sm[L.cof + q * npt + t] = G.cof[(size_t)(ORTH ? 2 * q : q) * npt + t] * iv;
+        sm[L.cof + q * npt + t] = G.cof[(size_t)(ORTH ? 2 * q : q) * npt + t];
     }
   }
   __syncthreads();
@@ -746,7 +748,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
     const int nph = (L.nx + 2) * (L.ny + 2), npt = L.nx * L.ny;
     for (int t = threadIdx.x; t < nph; t += kCoarseThreads) G.phi[(size_t)t * P + p] = sm[L.phi + t];
     if (l < g.lc)
-      for (int t = threadIdx.x; t < npt; t += kCoarseThreads) G.rhs[(size_t)t * P + p] = sm[L.rhs + t] * sm[L.c9 + t];
+      for (int t = threadIdx.x; t < npt; t += kCoarseThreads) G.rhs[(size_t)t * P + p] = sm[L.rhs + t];
   }
 }
 
