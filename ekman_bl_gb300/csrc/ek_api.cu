@@ -1524,8 +1524,11 @@ int ekgpu_mg_set_layout(ek_ctx *h, int level, int dir, int lanes, int seg) {
     std::vector<int> &u = dir ? PL.seg_x : PL.seg_y;
     if ((int)t.size() < PL.ngrid + 1) t.resize(PL.ngrid + 1, 0);
     if ((int)u.size() < PL.ngrid + 1) u.resize(PL.ngrid + 1, 0);
+    if ((int)PL.by_hand.size() < PL.ngrid + 1) PL.by_hand.resize(PL.ngrid + 1, 0);
     t[level] = lanes;
     u[level] = seg;
+    const int bit = 1 << dir;
+    PL.by_hand[level] = (lanes || seg) ? PL.by_hand[level] | bit : PL.by_hand[level] & ~bit;
     step_graphs_clear(c);  // captured with the old layouts
     return (int)EK_OK;
   });

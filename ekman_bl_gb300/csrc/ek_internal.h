@@ -168,8 +168,10 @@ struct MgPlan {
   size_t coarse_smem = 0;
   // mixed solver: layout of the line solves per level (index l = 1..ngrid)
   // and direction -- problems per block and rows per segment; 0 = the
-  // default rule (set by ekgpu_mg_autotune)
-  std::vector<int> lanes_y, lanes_x, seg_y, seg_x;
+  // default rule (set by ekgpu_mg_autotune and ekgpu_mg_set_layout); by_hand
+  // (bit 0 y-lines, bit 1 x-lines): the latter's, which also keeps the level
+  // out of the one-block launch
+  std::vector<int> lanes_y, lanes_x, seg_y, seg_x, by_hand;
 };
 
 // Kernel classes for the optional per-kernel timer (ekgpu_set_timing).

@@ -1791,12 +1791,9 @@ int tail_threads(const TailPlan &t, int nprob) {
 // (44 problems of 65 x 65: 12 launches a level and cycle of 5-9 us each, 27 us
 // in the block); with 342 problems a level of 65 x 97 in the block costs
 // 15.2 -> 16.2 ms a batch, and 33 x 49 gains 1% over leaving it out.  A level
-// whose line-solve layout was set by hand keeps its launches.
-bool layout_set(const MgPlan &PL, int l) {
-  for (const std::vector<int> *v : {&PL.lanes_y, &PL.lanes_x, &PL.seg_y, &PL.seg_x})
-    if (l < (int)v->size() && (*v)[l] > 0) return true;
-  return false;
-}
+// whose line-solve layout was set by hand keeps its launches; a tuned layout
+// serves the batches whose level is launched, and moves no level.
+bool layout_by_hand(const MgPlan &PL, int l) { return l < (int)PL.by_hand.size() && PL.by_hand[l]; }
 int tail_level(const MgPlan &PL, int nprob) {
   const int lth = thomas_levels(PL);
   if (lth == 0) return 0;
@@ -1804,7 +1801,7 @@ int tail_level(const MgPlan &PL, int nprob) {
   // (k_f_pline takes lines of at most 567 rows at 16 problems a block; longer
   // ones go one thread a line, in another order of operations)
   int top = lth;
-  while (top + 1 <= PL.ngrid && top + 1 <= kTailMax && !layout_set(PL, top + 1) && std::max(PL.lv[top].nx, PL.lv[top].ny) <= 567 &&
+  while (top + 1 <= PL.ngrid && top + 1 <= kTailMax && !layout_by_hand(PL, top + 1) && std::max(PL.lv[top].nx, PL.lv[top].ny) <= 567 &&
          tail_bytes_of(make_tail_plan(PL, top + 1, lth)) <= most)
     ++top;
   return top;
@@ -2225,6 +2222,7 @@ int mgfast_autotune(Ctx &c, int reps, std::string &report) {
   PL.lanes_x.assign(PL.ngrid + 1, 0);
   PL.seg_y.assign(PL.ngrid + 1, 0);
   PL.seg_x.assign(PL.ngrid + 1, 0);
+  PL.by_hand.assign(PL.ngrid + 1, 0);
   cudaEvent_t e0, e1;
   EK_CUDA(cudaEventCreate(&e0));
   EK_CUDA(cudaEventCreate(&e1));
@@ -2233,8 +2231,7 @@ int mgfast_autotune(Ctx &c, int reps, std::string &report) {
   try {
     // the Thomas levels of k_f_vtail have no line-solve launches to tune; the
     // levels above them that it takes by tail_level's rule are timed as
-    // launches but stay there (a layout would move them out)
-    const int ltop = tail_level(PL, nprob);
+    // launches, for the larger batches that run them so
     for (int l = std::max(2, thomas_levels(PL) + 1); l <= PL.ngrid; ++l) {
       const MgLevel &L = PL.lv[l - 1];
       for (int dir = 0; dir < 2; ++dir) {
@@ -2280,10 +2277,8 @@ int mgfast_autotune(Ctx &c, int reps, std::string &report) {
               best_ms = ms;
             }
           }
-        if (l > ltop) {
-          (xl ? PL.lanes_x : PL.lanes_y)[l] = best;
-          (xl ? PL.seg_x : PL.seg_y)[l] = best_seg;
-        }
+        (xl ? PL.lanes_x : PL.lanes_y)[l] = best;
+        (xl ? PL.seg_x : PL.seg_y)[l] = best_seg;
         report += std::string(first ? "" : ", ") + "{\"level\": " + std::to_string(l) + ", \"dir\": \"" +
                   (xl ? "x" : "y") + "\", \"n\": " + std::to_string(n) + ", \"us\": {" + row +
                   "}, \"lanes\": " + std::to_string(best) + ", \"seg\": " + std::to_string(best_seg) + "}";

@@ -338,8 +338,10 @@ int ekgpu_mg_levels(ek_ctx *ctx, int *ngrid, int *nx, int *ny, int cap);
  * no line-solve launches, so the autotuner times levels max(2, ltop+1)..ngrid
  * only and their layouts are not used.  Higher levels that fit a block's
  * shared memory run in the same launch, with the same results bit for bit as
- * 8-row segments give, while no layout is set for them: ekgpu_mg_set_layout
- * gives such a level its own launches, the autotuner leaves it where it is. */
+ * 8-row segments give, while no layout is set for them by hand:
+ * ekgpu_mg_set_layout gives such a level its own launches.  Which levels fit
+ * depends on the number of problems; a tuned layout is used by the batches
+ * that launch its level and moves none. */
 int ekgpu_mg_tail_levels(ek_ctx *ctx, int *ltop);
 
 /* ---- Learned initial guess of the per-kx Poisson problems -------------------
