@@ -32,11 +32,17 @@ def test_tuning_leaves_small_batches_alone():
     g.mg_autotune(reps=2)
     phi1, cyc1, n1 = solve()
     assert (cyc1, n1) == (cyc0, n0) and np.array_equal(phi0, phi1)
-    # by hand, the finest level has launches of its own, and none again with 0
+    # by hand, the finest level has launches of its own (in one direction
+    # alone, the other takes the tuned layout, whose segments may be shorter),
+    # and none again with 0
     top = len(g.mg_levels())
     g.mg_set_layout(top, 0, 16, 8)
+    assert solve()[2] > n0
+    g.mg_set_layout(top, 1, 16, 8)
     phi2, _, n2 = solve()
     assert n2 > n0 and np.array_equal(phi0, phi2)
     g.mg_set_layout(top, 0, 0, 0)
+    assert solve()[2] > n0
+    g.mg_set_layout(top, 1, 0, 0)
     phi3, _, n3 = solve()
     assert n3 == n0 and np.array_equal(phi0, phi3)
