@@ -1082,11 +1082,11 @@ void launch_c2r(Ctx &c, const C2rArgs &a) {
 
 namespace ek {
 void fft_init_attributes() {
-  static std::once_flag once;
-  std::call_once(once, [] {
-  smem_attributes<double>();
-  smem_attributes<float>();
-  smem_attributes<FF>();
+  static OncePerDevice once;
+  once(current_device(), [] {
+    smem_attributes<double>();
+    smem_attributes<float>();
+    smem_attributes<FF>();
   });
 }
 }  // namespace ek

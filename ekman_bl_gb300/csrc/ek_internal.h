@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/ekgpu.h"
+#include "ek_device.h"
 #include "ek_ffbits.h"
 
 namespace ek {
@@ -580,6 +581,12 @@ struct CudaError {
   std::string msg;
   explicit CudaError(std::string m) : msg(std::move(m)) {}
 };
+
+inline int current_device() {
+  int d = 0;
+  EK_CUDA(cudaGetDevice(&d));
+  return d;
+}
 
 inline void after_launch(Ctx &c) {
   c.launches++;

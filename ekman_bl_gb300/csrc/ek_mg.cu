@@ -28,8 +28,6 @@
 #include <algorithm>
 #include <cstdio>
 
-#include <mutex>
-
 #include "ek_internal.h"
 
 namespace ek {
@@ -977,8 +975,8 @@ void mg_null_mean(Ctx &c, double *phi_finest, int nprob, const double *kx2_dev) 
 // k_coarse's shared-memory limit, set once per process (outside any stream
 // capture; contexts stepping on several host threads may get here together).
 void mg_exact_attributes() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static OncePerDevice once;
+  once(current_device(), [] {
     // k_coarse: levels 1..lc take up to 112 KB (96 KB counted without c9), but a
     // level 1 larger than that is in it whatever its size, up to the most a
     // block can have

@@ -23,7 +23,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 
 #include "ek_internal.h"
 #include "ek_unet.h"
@@ -1171,10 +1170,10 @@ unsigned gsz(long n, int bs) {
 size_t img_bytes(int n, int h, int w, int c, size_t es) { return (size_t)n * (h + 2) * (w + 2) * c * es; }
 
 constexpr size_t kTcSmem = 220 * 1024;
-// One-time shared-memory limits (the same constants whichever thread is first)
+// Shared-memory limits, once a device (the same constants whichever thread is first)
 void kernel_limits() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static OncePerDevice once;
+  once(current_device(), [] {
     EK_CUDA(cudaFuncSetAttribute(k_conv_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
     EK_CUDA(cudaFuncSetAttribute(k_conv_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
     EK_CUDA(cudaFuncSetAttribute(k_conv_dw<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
@@ -1182,12 +1181,9 @@ void kernel_limits() {
   });
 }
 int sm_count() {
-  static const int n = [] {
-    int v = 0;
-    EK_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, 0));
-    return v;
-  }();
-  return n;
+  int v = 0;
+  EK_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, current_device()));
+  return v;
 }
 // The stage layout of k_conv_tc for a GEMM of K = 9 cin, N = cout on images g:
 // two stages when they fit, one otherwise.  plane: 16 bytes a pixel, 32 bytes
