@@ -999,6 +999,19 @@ struct TailPlan {
                                  // others the planes c1 c3 c5 c7 b (and c2 c4 c6 c8 unless orthogonal)
 };
 
+// Segments of a line of n rows in part_lines (k_f_pline's with 8-row segments),
+// and the floats of its exchange arrays for a colour's lines of both directions,
+// in a block of at most kTailMost threads
+constexpr int kPartSeg = 8;
+__host__ __device__ inline int part_segments(int n) {
+  const int k = (n + kPartSeg + 1) / (kPartSeg + 1);
+  return k > 1 ? k : 1;
+}
+int part_scratch(int nx, int ny) {
+  auto lines = [](int n, int colour) { return SH_N * part_segments(n) * std::min(kTailMost / part_segments(n), colour); };
+  return std::max(lines(nx, (ny + 1) / 2), lines(ny, (nx + 1) / 2));
+}
+
 TailPlan make_tail_plan(const MgPlan &PL, int ltop, int lth) {
   TailPlan t{};
   t.ltop = ltop;
@@ -1016,8 +1029,12 @@ TailPlan make_tail_plan(const MgPlan &PL, int ltop, int lth) {
     t.f[l] = fo;
     if (l < lth) fo += 4 * nx * ny;
   }
+  // the transfers' scratch, and part_lines' (the smaller one for every shape
+  // with sides of 6 to 700 points, by 11 floats at 7 x 9)
   t.scr = off;
-  off += (t.nx[ltop - 1] + 2) * (t.ny[ltop - 1] + 2);
+  int scr = (t.nx[ltop - 1] + 2) * (t.ny[ltop - 1] + 2);
+  for (int l = lth; l < ltop; ++l) scr = std::max(scr, part_scratch(t.nx[l], t.ny[l]));
+  off += scr;
   off = (off + 3) & ~3;  // the factor block is copied as float4
   t.fac0 = off;
   t.nfac = fo;
@@ -1284,14 +1301,14 @@ __device__ __forceinline__ void tail_coarse(const TailLv &L, int sweeps, bool or
 // The lines l0, l0 + lstep, ... (nline of them) of one colour by the whole
 // block, k_f_pline's partitioned solve operation for operation: thread (s, li)
 // owns segment s of line li, G lines at a time, sh the scratch of SH_N arrays
-// of K x G.  The level's coefficients and the problem's diagonal are staged in
+// of K x G (part_scratch).  The level's coefficients and the problem's diagonal are staged in
 // shared memory: read from L2, a colour's 110 KB (65 x 65) at an SM's share of
 // the L2 bandwidth took longer than the solve.
 template <bool XL, bool ORTH>
 __device__ __forceinline__ void part_lines(const TailLv &L, float *sh, int l0, int lstep, int nline) {
-  constexpr int SEG = 8;
+  constexpr int SEG = kPartSeg;
   const int nx = L.nx, ny = L.ny, n = XL ? nx : ny, sj = nx + 2, npt = nx * ny;
-  const int K = max(1, (n + SEG + 1) / (SEG + 1));
+  const int K = part_segments(n);
   const int mb = (n - K + 1) / K, me = (n - K + 1) - mb * K;
   const int G = min((int)blockDim.x / K, nline);
   const int s0 = (int)threadIdx.x / G, li = (int)threadIdx.x - s0 * G;
