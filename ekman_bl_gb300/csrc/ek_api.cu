@@ -980,8 +980,7 @@ int ekgpu_set_metrics(ek_ctx *h, const ek_metrics *m) {
       EK_CUDA(cudaMemcpy(c.mg_z, z.data(), sizeof(double) * z.size(), cudaMemcpyHostToDevice));
     }
     // the levels that one block of k_coarse holds: level 1, and those above it
-    // while their phi, rhs, 1/c9 and couplings and the scratch fit 96 KB (the
-    // kernel keeps c9 as well)
+    // while their phi, rhs, 1/c9 and couplings and the scratch fit 96 KB
     const int ncof = P.orth ? 4 : 8;
     P.lc = 1;
     for (int l = 1; l <= P.ngrid; ++l) {

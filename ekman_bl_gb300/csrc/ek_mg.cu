@@ -501,7 +501,7 @@ __global__ void k_check_finish(MgDev g, int iter, int last) {
 // Coarse levels 1..lc: one CTA per problem, everything in shared memory.
 struct CoarseLv {
   int nx, ny;
-  int phi, rhs, inv9, c9, cof;  // offsets (doubles) into shared memory
+  int phi, rhs, inv9, cof;  // offsets (doubles) into shared memory
 };
 struct CoarseArgs {
   MgDev g;
@@ -520,7 +520,7 @@ constexpr int kCoarseThreads = 256;
 // however many of its lanes work (measured), so the points are packed over
 // the threads, and while the phase fits four warps that way two lanes share a
 // point's couplings and add their halves.  (One lane a point: ten dependent
-// operations, 298 us a launch on 64 x 129 x 97 sheared; now 187.  With the
+// operations, 298 us a launch on 64 x 129 x 97 sheared; now 183.  With the
 // right-hand side and the couplings divided by c9 beforehand a point takes one
 // operation less, 178 us, but each such quotient is rounded: on grids of one
 // block, solved to convergence, up to four times the error against 64-bit
@@ -599,32 +599,48 @@ __device__ __forceinline__ void c_relax(const CoarseArgs &A, double *sm, int lev
 }
 
 template <bool ORTH>
-__device__ __forceinline__ void c_restrict(const CoarseArgs &A, double *sm, int level) {
+__device__ __forceinline__ void c_restrict(const CoarseArgs &A, double *sm, int level, double kx2) {
   const CoarseLv &F = A.lv[level - 1], &C = A.lv[level - 2];
   const int nx = F.nx, ny = F.ny, ncx = C.nx, ncy = C.ny;
   const double *phi = sm + F.phi, *rhs = sm + F.rhs, *cf = sm + F.cof;
   double *scr = sm + A.scr;
   const int npt = nx * ny, sj = nx + 2;
-  const double *c9 = sm + F.c9;
-  for (int t = threadIdx.x; t < nx * ny; t += blockDim.x) {
-    const int i = 1 + t % nx, j = 1 + t / nx;
-    const double *ph = phi + j * sj + i;
-    double s = cf[t] * ph[1];
-    if (ORTH) {
-      s = s + cf[npt + t] * ph[sj];
-      s = s + cf[2 * npt + t] * ph[-1];
-      s = s + cf[3 * npt + t] * ph[-sj];
-    } else {
-      s = s + cf[npt + t] * ph[1 + sj];
-      s = s + cf[2 * npt + t] * ph[sj];
-      s = s + cf[3 * npt + t] * ph[sj - 1];
-      s = s + cf[4 * npt + t] * ph[-1];
-      s = s + cf[5 * npt + t] * ph[-1 - sj];
-      s = s + cf[6 * npt + t] * ph[-sj];
-      s = s + cf[7 * npt + t] * ph[1 - sj];
+  // c9 from its kx-independent parts, which all problems share, in L2: kept in
+  // shared memory it leaves an SM two blocks for three on many grids (684
+  // problems of 97 x 65: 13.3 ms a step's coarse levels against 8.2; where the
+  // blocks fit either way 3% in its favour).  Loads for U points go out together.
+  const double *gd = A.g.lv[level - 1].cof + 8 * npt;
+  constexpr int U = 4;
+  for (int t0 = threadIdx.x; t0 < npt; t0 += U * kCoarseThreads) {
+    double c9[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = min(t0 + u * kCoarseThreads, npt - 1);
+      c9[u] = ((-kx2 * gd[2 * npt + t]) - gd[t]) + gd[npt + t];
     }
-    s = s + c9[t] * ph[0];
-    scr[j * sj + i] = rhs[t] - s;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * kCoarseThreads;
+      if (t >= npt) break;
+      const int i = 1 + t % nx, j = 1 + t / nx;
+      const double *ph = phi + j * sj + i;
+      double s = cf[t] * ph[1];
+      if (ORTH) {
+        s = s + cf[npt + t] * ph[sj];
+        s = s + cf[2 * npt + t] * ph[-1];
+        s = s + cf[3 * npt + t] * ph[-sj];
+      } else {
+        s = s + cf[npt + t] * ph[1 + sj];
+        s = s + cf[2 * npt + t] * ph[sj];
+        s = s + cf[3 * npt + t] * ph[sj - 1];
+        s = s + cf[4 * npt + t] * ph[-1];
+        s = s + cf[5 * npt + t] * ph[-1 - sj];
+        s = s + cf[6 * npt + t] * ph[-sj];
+        s = s + cf[7 * npt + t] * ph[1 - sj];
+      }
+      s = s + c9[u] * ph[0];
+      scr[j * sj + i] = rhs[t] - s;
+    }
   }
   __syncthreads();
   const int ix = (ncx == nx) ? 0 : 1, jy = (ncy == ny) ? 0 : 1;
@@ -702,6 +718,9 @@ __device__ __forceinline__ void c_prolong(const CoarseArgs &A, double *sm, int l
   __syncthreads();
 }
 
+// Levels 1..lc fit 96 KB; a level 1 beyond that runs here all the same, up to this.
+constexpr size_t kCoarseSmem = 200 * 1024;
+
 template <bool ORTH>
 __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
   extern __shared__ double sm[];
@@ -709,8 +728,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
   const int p = blockIdx.x;
   if (*g.alldone || g.done[p]) return;
   const int P = g.P;
-  // load every coarse level (phi with ghosts, rhs, 1/c9, c9, couplings)
-  const double kx2 = g.kx2[p];
+  // load every coarse level (phi with ghosts, rhs, 1/c9, couplings)
   for (int l = 1; l <= g.lc; ++l) {
     const CoarseLv &L = A.lv[l - 1];
     const LvDev &G = g.lv[l - 1];
@@ -721,7 +739,6 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
     for (int t = threadIdx.x; t < npt; t += kCoarseThreads) {
       sm[L.rhs + t] = G.rhs[(size_t)t * P + p];
       sm[L.inv9 + t] = G.inv9[(size_t)t * P + p];
-      sm[L.c9 + t] = ((-kx2 * G.cof[(size_t)10 * npt + t]) - G.cof[(size_t)8 * npt + t]) + G.cof[(size_t)9 * npt + t];
       // c1, c3, c5, c7 or c1..c8
 #pragma unroll
       for (int q = 0; q < (ORTH ? 4 : 8); ++q)
@@ -734,7 +751,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarseArgs A) {
   for (int o = 0; o < A.nops; ++o) {
     const MgOp op = A.ops[o];
     if (op.kind == OP_RELAX) c_relax<ORTH>(A, sm, op.level, op.count, stale[op.level - 1]);
-    else if (op.kind == OP_RESTRICT) c_restrict<ORTH>(A, sm, op.level);
+    else if (op.kind == OP_RESTRICT) c_restrict<ORTH>(A, sm, op.level, g.kx2[p]);
     else if (op.kind == OP_COR2) c_prolong(A, sm, op.level, 0, stale[op.level - 1]);
     else if (op.kind == OP_PROLONG) c_prolong(A, sm, op.level + 1, 1, stale[op.level]);
   }
@@ -977,11 +994,8 @@ void mg_null_mean(Ctx &c, double *phi_finest, int nprob, const double *kx2_dev) 
 void mg_exact_attributes() {
   static OncePerDevice once;
   once(current_device(), [] {
-    // k_coarse: levels 1..lc take up to 112 KB (96 KB counted without c9), but a
-    // level 1 larger than that is in it whatever its size, up to the most a
-    // block can have
-    EK_CUDA(cudaFuncSetAttribute(k_coarse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemSM - kSmemKept)));
-    EK_CUDA(cudaFuncSetAttribute(k_coarse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemSM - kSmemKept)));
+    EK_CUDA(cudaFuncSetAttribute(k_coarse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
+    EK_CUDA(cudaFuncSetAttribute(k_coarse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
     EK_CUDA(cudaFuncSetAttribute(k_relax_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRelaxSmem));
   });
 }
@@ -1033,7 +1047,6 @@ void mg_exact_enqueue(Ctx &c, MgWork &w, int nprob, const double *kx2_dev, int m
     A.lv[l - 1].phi = off; off += (L.nx + 2) * (L.ny + 2);
     A.lv[l - 1].rhs = off; off += L.nx * L.ny;
     A.lv[l - 1].inv9 = off; off += L.nx * L.ny;
-    A.lv[l - 1].c9 = off; off += L.nx * L.ny;
     A.lv[l - 1].cof = off; off += ncof * L.nx * L.ny;
     maxph = std::max(maxph, (L.nx + 2) * (L.ny + 2));
   }
