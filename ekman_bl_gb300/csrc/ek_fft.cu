@@ -255,46 +255,61 @@ __device__ __forceinline__ T flux_gen(const FluxG12<T> &g, T f, T fkp, T fkm, T 
   s2 = -s2 + g.qv * (g.c * (fpp + fkp - fmp - fkm) - g.d * (fkp + fpm - fkm - fmm));
   return s1 + s2;
 }
-// Two consecutive values in the arithmetic type: one 8-byte load of an FP32
-// plane (a plane's lines start on even elements)
+// One or two consecutive values in the arithmetic type: two in one 8-byte load
+// of an FP32 plane (a plane's lines start on even elements)
+template <typename T> struct One {
+  T x;
+};
 template <typename T> struct Two {
   T x, y;
 };
-template <typename T> __device__ __forceinline__ Two<T> two(const float *p) {
-  const float2 v = *reinterpret_cast<const float2 *>(p);
-  return Two<T>{(T)(double)v.x, (T)(double)v.y};
+template <typename T, typename P> __device__ __forceinline__ void ld_pts(One<T> &v, const P *p) { v.x = (T)(double)p[0]; }
+template <typename T> __device__ __forceinline__ void ld_pts(Two<T> &v, const float *p) {
+  const float2 w = *reinterpret_cast<const float2 *>(p);
+  v.x = (T)(double)w.x, v.y = (T)(double)w.y;
 }
-template <typename T> __device__ __forceinline__ Two<T> two(const double *p) { return Two<T>{(T)p[0], (T)p[1]}; }
-// The flux at points c and c + 1, its loads apart from its value so that
-// several pairs' loads can go out together; b is U2b, followed in memory by U3b
+template <typename T> __device__ __forceinline__ void ld_pts(Two<T> &v, const double *p) { v.x = (T)p[0], v.y = (T)p[1]; }
+template <typename G, typename P> __device__ __forceinline__ G pts(const P *p) {
+  G v;
+  ld_pts(v, p);
+  return v;
+}
+// The flux at the points from c on, its loads apart from its value so that
+// several groups' loads can go out together; b is U2b, followed in memory by U3b
 // (see the launch).
-template <typename T> struct FluxIn {
-  Two<T> f, kp, km, jp, jm, u2, u2p, u3, u3p, pp, pm, mp, mm;
+template <typename G> struct FluxIn {
+  G f, kp, km, jp, jm, u2, u2p, u3, u3p, pp, pm, mp, mm;
 };
-template <typename T, bool ORTH, typename P>
-__device__ __forceinline__ FluxIn<T> flux_load(const Dims &d, size_t c, const P *F, const P *U2b) {
+template <typename G, bool ORTH, typename P>
+__device__ __forceinline__ FluxIn<G> flux_load(const Dims &d, size_t c, const P *F, const P *U2b) {
   const size_t sK = d.LDX, sJ = (size_t)d.LDX * d.NZ2;
   const P *U3b = U2b + d.nphys();
-  FluxIn<T> v;
-  v.f = two<T>(F + c), v.kp = two<T>(F + c + sK), v.km = two<T>(F + c - sK);
-  v.jp = two<T>(F + c + sJ), v.jm = two<T>(F + c - sJ);
-  v.u2 = two<T>(U2b + c), v.u2p = two<T>(U2b + c + sJ), v.u3 = two<T>(U3b + c), v.u3p = two<T>(U3b + c + sK);
+  FluxIn<G> v;
+  v.f = pts<G>(F + c), v.kp = pts<G>(F + c + sK), v.km = pts<G>(F + c - sK);
+  v.jp = pts<G>(F + c + sJ), v.jm = pts<G>(F + c - sJ);
+  v.u2 = pts<G>(U2b + c), v.u2p = pts<G>(U2b + c + sJ), v.u3 = pts<G>(U3b + c), v.u3p = pts<G>(U3b + c + sK);
   if constexpr (!ORTH) {
-    v.pp = two<T>(F + c + sK + sJ), v.pm = two<T>(F + c + sK - sJ);
-    v.mp = two<T>(F + c - sK + sJ), v.mm = two<T>(F + c - sK - sJ);
+    v.pp = pts<G>(F + c + sK + sJ), v.pm = pts<G>(F + c + sK - sJ);
+    v.mp = pts<G>(F + c - sK + sJ), v.mm = pts<G>(F + c - sK - sJ);
   }
   return v;
 }
-template <bool ORTH, typename T>
-__device__ __forceinline__ Two<T> flux_value(const FluxG12<T> &g, const FluxIn<T> &v) {
+template <bool ORTH, typename T, typename G>
+__device__ __forceinline__ G flux_value(const FluxG12<T> &g, const FluxIn<G> &v) {
+  G r;
   if constexpr (ORTH)
-    return Two<T>{flux_orth(v.f.x, v.kp.x, v.km.x, v.jp.x, v.jm.x, v.u2.x, v.u2p.x, v.u3.x, v.u3p.x),
-                  flux_orth(v.f.y, v.kp.y, v.km.y, v.jp.y, v.jm.y, v.u2.y, v.u2p.y, v.u3.y, v.u3p.y)};
+    r.x = flux_orth(v.f.x, v.kp.x, v.km.x, v.jp.x, v.jm.x, v.u2.x, v.u2p.x, v.u3.x, v.u3p.x);
   else
-    return Two<T>{flux_gen(g, v.f.x, v.kp.x, v.km.x, v.jp.x, v.jm.x, v.pp.x, v.pm.x, v.mp.x, v.mm.x, v.u2.x, v.u2p.x,
-                           v.u3.x, v.u3p.x),
-                  flux_gen(g, v.f.y, v.kp.y, v.km.y, v.jp.y, v.jm.y, v.pp.y, v.pm.y, v.mp.y, v.mm.y, v.u2.y, v.u2p.y,
-                           v.u3.y, v.u3p.y)};
+    r.x = flux_gen(g, v.f.x, v.kp.x, v.km.x, v.jp.x, v.jm.x, v.pp.x, v.pm.x, v.mp.x, v.mm.x, v.u2.x, v.u2p.x, v.u3.x,
+                   v.u3p.x);
+  if constexpr (std::is_same_v<G, Two<T>>) {
+    if constexpr (ORTH)
+      r.y = flux_orth(v.f.y, v.kp.y, v.km.y, v.jp.y, v.jm.y, v.u2.y, v.u2p.y, v.u3.y, v.u3p.y);
+    else
+      r.y = flux_gen(g, v.f.y, v.kp.y, v.km.y, v.jp.y, v.jm.y, v.pp.y, v.pm.y, v.mp.y, v.mm.y, v.u2.y, v.u2p.y, v.u3.y,
+                     v.u3p.y);
+  }
+  return r;
 }
 // The same along one x-line, point n to put(n, value), for the FP64 kernel.
 // The choice is made for a whole line at once, so that either loop's loads
@@ -321,11 +336,11 @@ __device__ __forceinline__ void flux_line(Put put, const FftConst &fc, int k, in
   }
 }
 
-// The FP32 register form asks for 8 blocks an SM (64 registers, a 16-byte
-// spill; 72 registers left 7): the step's forward transforms 10.6 -> 9.8 ms
+// The FP32 register form asks for 8 blocks an SM (64 registers, spills of 8 to
+// 48 bytes; 72 registers left 7): the step's forward transforms 10.6 -> 9.8 ms
 // on 512 x 385 x 257.  A minimum of 0 leaves the other forms' allocation
 // as the compiler chooses it.
-template <typename T, int E>
+template <typename T, int E, bool SHORT = false>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0) ? 8 : 0)
     k_r2c(FftConst fc, R2cArgs args) {
   using V = typename Cx<T>::V;
@@ -346,41 +361,51 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
   constexpr bool kF = sizeof(T) == 4;
   const bool fin = kF && args.af != nullptr;  // FP32 copies of the inputs
   // Points go two at a time, and the loads of U pairs go out before any of them
-  // is used: a load a turn leaves the memory waiting.
+  // is used: a load a turn leaves the memory waiting.  SHORT (NX <= 32): a point
+  // a lane, as pairs would leave half the warp idle.
+  using G = std::conditional_t<SHORT, One<T>, Two<T>>;
+  constexpr int W = SHORT ? 1 : 2;
+  const int items = SHORT ? 2 * M : M;
   auto batch = [&](auto U_, auto load, auto use) {
-    constexpr int U = decltype(U_)::value, B = (E > 0 && E < U) ? E : U;
-    for (int m0 = lane; m0 < M; m0 += 32 * B) {
+    constexpr int U = SHORT ? 1 : decltype(U_)::value, B = (E > 0 && E < U) ? E : U;
+    for (int m0 = lane; m0 < items; m0 += 32 * B) {
       decltype(load(0)) v[B];
 #pragma unroll
       for (int u = 0; u < B; ++u)
-        if (E > 0 || m0 + 32 * u < M) v[u] = load(m0 + 32 * u);
+        if (E > 0 || m0 + 32 * u < items) v[u] = load(m0 + 32 * u);
 #pragma unroll
       for (int u = 0; u < B; ++u)
-        if (E > 0 || m0 + 32 * u < M) use(m0 + 32 * u, v[u]);
+        if (E > 0 || m0 + 32 * u < items) use(m0 + 32 * u, v[u]);
     }
   };
   constexpr std::integral_constant<int, 4> U4{};
-  auto store = [&](int m, Two<T> v) { z[m] = Cx<T>::make(v.x, v.y); };
+  auto put = [&](V *y, int m, const G &v) {
+    if constexpr (SHORT) reinterpret_cast<T *>(y)[m] = v.x;
+    else y[m] = Cx<T>::make(v.x, v.y);
+  };
+  auto store = [&](int m, const G &v) { put(z, m, v); };
   auto flux = [&](V *y, auto *F, auto *b, double visc) {
     const FluxG12<T> g(fc, k, j, visc);
     auto line = [&](auto ORTH) {
       constexpr bool O = decltype(ORTH)::value;
       // a general pair is 26 values, an orthogonal one 18
       constexpr std::integral_constant<int, (kF && O) ? 2 : 1> UF{};
-      batch(UF, [&](int m) { return flux_load<T, O>(d, base + 2 * m, F, b); },
-            [&](int m, const FluxIn<T> &v) {
-              const Two<T> f = flux_value<O>(g, v);
-              y[m] = Cx<T>::make(f.x, f.y);
-            });
+      batch(UF, [&](int m) { return flux_load<G, O>(d, base + W * m, F, b); },
+            [&](int m, const FluxIn<G> &v) { put(y, m, flux_value<O>(g, v)); });
     };
     if (fc.orth) line(std::true_type{});
     else line(std::false_type{});
   };
   auto add = [&](V *y, auto *x, T es) {
-    batch(U4, [&](int m) { return two<T>(x + base + 2 * m); },
-          [&](int m, Two<T> v) {
-            const V o = y[m];
-            y[m] = Cx<T>::make(o.x + es * v.x, o.y + es * v.y);
+    batch(U4, [&](int m) { return pts<G>(x + base + W * m); },
+          [&](int m, const G &v) {
+            if constexpr (SHORT) {
+              T &o = reinterpret_cast<T *>(y)[m];
+              o = o + es * v.x;
+            } else {
+              const V o = y[m];
+              y[m] = Cx<T>::make(o.x + es * v.x, o.y + es * v.y);
+            }
           });
   };
   if (args.pro == PRO_LOAD) {
@@ -390,24 +415,35 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
       pairs = args.alo != nullptr;
       if (pairs)
         batch(U4, [&](int m) {
-          const float2 h = *reinterpret_cast<const float2 *>(args.af + base + 2 * m);
-          const float2 l = *reinterpret_cast<const float2 *>(args.alo + base + 2 * m);
-          return Two<T>{FF(h.x, l.x), FF(h.y, l.y)};
+          G v;
+          if constexpr (SHORT) {
+            v.x = FF(args.af[base + m], args.alo[base + m]);
+          } else {
+            const float2 h = *reinterpret_cast<const float2 *>(args.af + base + 2 * m);
+            const float2 l = *reinterpret_cast<const float2 *>(args.alo + base + 2 * m);
+            v.x = FF(h.x, l.x), v.y = FF(h.y, l.y);
+          }
+          return v;
         }, store);
     }
     // fin: an FP32 field (the increment of the state)
     if (!pairs) {
-      if (fin) batch(U4, [&](int m) { return two<T>(args.af + base + 2 * m); }, store);
-      else batch(U4, [&](int m) { return two<T>(args.a + base + 2 * m); }, store);
+      if (fin) batch(U4, [&](int m) { return pts<G>(args.af + base + W * m); }, store);
+      else batch(U4, [&](int m) { return pts<G>(args.a + base + W * m); }, store);
     }
   } else if (args.pro == PRO_PROD) {
     const T jac = from_f64<T>(fc.m.jac[d.m2(k, j)]);
     auto prod = [&](auto *a, auto *b) {
       struct In {
-        Two<T> a, b;
+        G a, b;
       };
-      batch(U4, [&](int m) { return In{two<T>(a + base + 2 * m), two<T>(b + base + 2 * m)}; },
-            [&](int m, const In &v) { z[m] = Cx<T>::make(jac * v.a.x * v.b.x, jac * v.a.y * v.b.y); });
+      batch(U4, [&](int m) { return In{pts<G>(a + base + W * m), pts<G>(b + base + W * m)}; },
+            [&](int m, const In &v) {
+              G r;
+              r.x = jac * v.a.x * v.b.x;
+              if constexpr (!SHORT) r.y = jac * v.a.y * v.b.y;
+              put(z, m, r);
+            });
     };
     if (fin) prod(args.af, args.bf);
     else prod(args.a, args.b);
@@ -492,7 +528,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
     }
     }
   };
-  constexpr int UE = 3;
+  constexpr int UE = SHORT ? 1 : 3;
   for (int k0 = lane; k0 <= NKX; k0 += 32 * UE) {
     cplx_t o[UE];
 #pragma unroll
@@ -506,7 +542,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, (sizeof(T) == 4 && E > 0)
     for (int kk = NKX + 1 + lane; kk <= d.NX2P; kk += 32) dst[kk] = cplx_t{0.0, 0.0};
 }
 
-template <typename T, int E>
+template <typename T, int E, bool SHORT = false>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_c2r(FftConst fc, C2rArgs args) {
   using V = typename Cx<T>::V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -530,7 +566,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_c2r(FftConst fc, C2rArg
   // lane merges the pair (k, M-k) in place (X_M = 0: k = 0 pairs with zero).
   // Loads go out four modes a lane at a time, before any of them is used: a
   // load a turn had 16 KB an SM on the way, and 3 TB/s is what that gives.
-  constexpr int U = (E > 0 && E < 4) ? E : 4;
+  constexpr int U = SHORT ? 1 : (E > 0 && E < 4) ? E : 4;
   for (int k0 = lane; k0 < M; k0 += 32 * U) {
     cplx_t v[U];
 #pragma unroll
@@ -945,6 +981,9 @@ bool launch64(int nk, int nj, cudaStream_t s, const FftConst &fc, const R2cArgs 
 // 5.55, at the cost of resident blocks); 128 x 129 x 97 0.63 -> 0.56 and 0.66 ->
 // 0.60; 64 x 65 x 65 0.243 -> 0.233 and 0.401 -> 0.388; the float-float
 // inverse of 256 x 193 x 129 2.18 -> 2.02.
+// Lines of NX <= 32 keep a point and a mode a lane: pairs leave half a warp idle.
+// Two steps of 32 x 257 x 193, forward 2.90 with pairs, 2.42 so; with LES 3.88
+// and 3.18; 16 x 257 x 193 2.57 and 2.17, 3.41 and 2.79.
 template <typename T>
 void run_r2c(dim3 grid, size_t smem, cudaStream_t s, const FftConst &fc, const R2cArgs &a) {
   const unsigned nt = 32 * kWarpsPerBlock;
@@ -958,7 +997,8 @@ void run_r2c(dim3 grid, size_t smem, cudaStream_t s, const FftConst &fc, const R
       default: break;
     }
   }
-  k_r2c<T, 0><<<grid, nt, smem, s>>>(fc, a);
+  if (fc.M <= 16) k_r2c<T, 0, true><<<grid, nt, smem, s>>>(fc, a);
+  else if constexpr (!std::is_same_v<T, float>) k_r2c<T, 0><<<grid, nt, smem, s>>>(fc, a);
 }
 template <typename T>
 void run_c2r(dim3 grid, size_t smem, cudaStream_t s, const FftConst &fc, const C2rArgs &a) {
@@ -973,13 +1013,16 @@ void run_c2r(dim3 grid, size_t smem, cudaStream_t s, const FftConst &fc, const C
       default: break;
     }
   }
-  k_c2r<T, 0><<<grid, nt, smem, s>>>(fc, a);
+  if (fc.M <= 16) k_c2r<T, 0, true><<<grid, nt, smem, s>>>(fc, a);
+  else if constexpr (!std::is_same_v<T, float>) k_c2r<T, 0><<<grid, nt, smem, s>>>(fc, a);
 }
 template <typename T>
 void smem_attributes() {
   const int b = 96 * 1024;
-  EK_CUDA(cudaFuncSetAttribute(k_r2c<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-  EK_CUDA(cudaFuncSetAttribute(k_c2r<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+  if constexpr (!std::is_same_v<T, float>) {
+    EK_CUDA(cudaFuncSetAttribute(k_r2c<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    EK_CUDA(cudaFuncSetAttribute(k_c2r<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+  }
   if constexpr (std::is_same_v<T, double>) {
     EK_CUDA(cudaFuncSetAttribute(k_r2c64<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
     EK_CUDA(cudaFuncSetAttribute(k_r2c64<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
