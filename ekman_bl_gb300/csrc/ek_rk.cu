@@ -2505,7 +2505,8 @@ int finish_divergence(Ctx &c, double *div_out) {
 }  // namespace ek
 
 namespace ek {
-// The RK kernels use the default shared-memory limit.
+// The increment form's tiles are the RK kernels that need more than the default
+// shared memory; called for each context, on its device.
 void rk_init_attributes() {
   const int most = (int)adi_tile_smem(kAdiTileRows);
   EK_CUDA(cudaFuncSetAttribute(k_adi_inc_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));

@@ -66,7 +66,6 @@ struct ConvArgs {
   const float *dz;      // FP32 [.. cout] with border
   float *dx1, *dx2;     // FP32 [.. c1], [.. c2] with border
   const unsigned short *m1, *m2;  // ReLU masks (the activations x1, x2), or null
-  int acc1, acc2;       // accumulate into dx1 / dx2 instead of storing
   // weight-gradient pass
   const unsigned short *dzb;  // dZ rounded to BF16, bordered (the tensor-core passes' operand)
   unsigned short *dxb1, *dxb2;  // BF16 copies of dx1 / dx2 (null: none)
@@ -172,11 +171,11 @@ __device__ __forceinline__ void epilogue(const ConvArgs &a, long m, int nn, floa
     if (nn < a.c1) {
       const size_t q = a.g.at(n, y, x, a.c1) + nn;
       if (a.m1 && !(bf2f(a.m1[q]) > 0.f)) v = 0.f;
-      a.dx1[q] = a.acc1 ? a.dx1[q] + v : v;
+      a.dx1[q] = v;
     } else {
       const size_t q = a.g.at(n, y, x, a.c2) + (nn - a.c1);
       if (a.m2 && !(bf2f(a.m2[q]) > 0.f)) v = 0.f;
-      a.dx2[q] = a.acc2 ? a.dx2[q] + v : v;
+      a.dx2[q] = v;
     }
   } else {
     atomicAdd(&a.dw[(size_t)m * 9 * a.cin + nn], v);
