@@ -545,8 +545,8 @@ def run_gpu(args):
             roof = {"bound": "hbm", "kernel": name, "achieved": round(achieved, 1), "peak": peak,
                     "unit": "GB/s", "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
                     "traffic": traffic, "traffic_source": tsrc,
-                    "traffic_note": (f"DRAM bytes per algorithmic byte ({ratio}) of one finest-level sweep of the "
-                                     f"class's kernel, measured with ncu on the NX=128 case (fields above L2), "
+                    "traffic_note": (f"DRAM bytes per algorithmic byte ({ratio}) of a cycle's two finest-level sweeps "
+                                     f"with the class's kernel, measured with ncu on the NX=128 case (fields above L2), "
                                      f"times this class's algorithmic bytes per launch") if ratio else None,
                     "algorithmic_bytes_per_launch": int(dbytes / dcnt),
                     "avg_launch_us": round(dms * 1000.0 / dcnt, 3), "launches_per_step": dcnt,

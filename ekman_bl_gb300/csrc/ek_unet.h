@@ -39,8 +39,8 @@ class UNet {
   const float *grads() const { return grad_; }
   long launches() const { return launches_; }
   double forward_flops(int n) const;  // 2 x multiply-adds of the convolutions
-  // the forward convolutions whose channel counts allow it on the tcgen05
-  // kernel (default), else all on the mma.sync one
+  // the layers whose channel counts allow it on the tensor-core kernels, in
+  // every pass (default), else all on the element-wise mma.sync one
   void set_tcgen05(bool on) { tc_ = on; }
   bool tcgen05() const { return tc_; }
   // 1 when a tcgen05 convolution's bounded wait ran out (sticky); reads the

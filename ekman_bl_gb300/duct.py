@@ -583,8 +583,8 @@ class UNet:
                                                C.c_void_p(stream or 0)))
 
     def set_tcgen05(self, on: bool):
-        """Forward convolutions on the tcgen05 tensor-core kernel where their
-        channel counts allow it (the default), or all on the mma.sync one."""
+        """Convolutions on the tensor-core kernels where their channel counts
+        allow it (the default), or all on the element-wise mma.sync one."""
         self._check(self._L.ekgpu_unet_set_tcgen05(self._h, int(bool(on))))
 
     def train_step(self, x_ptr: int, t_ptr: int, n: int, hv: int, wv: int, lr: float,

@@ -366,16 +366,19 @@ int ekgpu_unet_set_params(ek_unet *net, const float *params);   /* host; resets 
 int ekgpu_unet_get_params(ek_unet *net, float *params);         /* host               */
 /* y[n][h][w] = net(x[n][h][w][cin]); device pointers; stream may be NULL */
 int ekgpu_unet_forward(ek_unet *net, const float *x_dev, int n, float *y_dev, void *stream);
-/* Forward convolutions with cin and cout multiples of 16 run on the tcgen05
- * tensor-core kernel (on by default); 0 puts every layer on the mma.sync
- * kernel.  No counterpart in the reference (method tuning). */
+/* Convolutions with cin and cout multiples of 16 run on the tensor-core
+ * kernels, forward and input gradient on tcgen05 (on by default; networks of
+ * 16 or 32 channels, EK_ERR_CUDA for 48 and 64); 0 puts every layer on the
+ * element-wise mma.sync kernel.  No counterpart in the reference (method tuning). */
 int ekgpu_unet_set_tcgen05(ek_unet *net, int on);
 /* one Adam step (beta 0.9/0.999, eps 1e-8) on the mean-square error against
- * t[n][h][w] over the top-left hv x wv pixels of each image */
+ * t[n][h][w] over the top-left hv x wv pixels of each image; on
+ * EK_ERR_TIMEOUT parameters and moments are as before, *loss is not written */
 int ekgpu_unet_train_step(ek_unet *net, const float *x_dev, const float *t_dev, int n, int hv, int wv,
                           double lr, double *loss, void *stream);
 /* forward and backward without an update: loss, prediction (y_dev may be
- * NULL) and the parameter gradient copied to grad_host (may be NULL) */
+ * NULL) and the parameter gradient copied to grad_host (may be NULL); on
+ * EK_ERR_TIMEOUT neither *loss nor grad_host is written */
 int ekgpu_unet_gradient(ek_unet *net, const float *x_dev, const float *t_dev, int n, int hv, int wv,
                         double *loss, float *y_dev, float *grad_host, void *stream);
 /* Image geometry of the guess at averaging factor f: the finest multigrid
